@@ -372,6 +372,9 @@ static float recip_rn(float f) {
     return best;
 }
 
+// RN(1/f - r) for r = RN(1/f): 1 - r f is exact in double.
+static float recip_lo(float f, float r) { return (float)((1.0 - (double)r * (double)f) / (double)f); }
+
 // TMA maps of a pitched field: x boxes [32 lines][32 elements] with the 128-byte swizzle over
 // (P, N*N); y boxes [32 elements][32 lines] over (P, N, N); z boxes over (P*N, N).
 static gell_status make_tensor_maps(gell_ctx* c, Substrate& sub) {
@@ -452,7 +455,7 @@ gell_status gell_substrate_add(gell_ctx* c, const gell_substrate* s, int* index_
         for (int j = 0; j < Na; ++j) {
             const bool in = j >= 1 && j <= c->g.N - 2;
             const float rj = efr[2 * c->g.N + j];
-            frs[j] = in ? make_float4(sub.F[j], rj, sub.side, sub.side * rj) : make_float4(1.f, 1.f, 0.f, 0.f);
+            frs[j] = in ? make_float4(sub.F[j], rj, sub.side, recip_lo(sub.F[j], rj)) : make_float4(1.f, 1.f, 0.f, 0.f);
         }
         const int N = c->g.N;
         const uint32_t eb = bits_of(sub.E[N - 2]), fb2 = bits_of(sub.F[N - 2]);
@@ -462,6 +465,7 @@ gell_status gell_substrate_add(gell_ctx* c, const gell_substrate* s, int* index_
             if (uni) sub.uniform_groups |= 1u << g;
         }
         sub.conv_R = recip_rn(sub.F[N - 2]);
+        sub.conv_L = recip_lo(sub.F[N - 2], sub.conv_R);
         GELL_CUDA(c, cudaMalloc(&sub.FRS, frs.size() * sizeof(float4)));
         GELL_CUDA(c, cudaMemcpyAsync(sub.FRS, frs.data(), frs.size() * sizeof(float4), cudaMemcpyHostToDevice,
                                      c->stream));

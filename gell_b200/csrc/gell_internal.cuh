@@ -55,8 +55,8 @@ struct Substrate {
     float* p = nullptr;     // field, pitched
     float* rate = nullptr;  // uptake map, pitched; nonzero only on flagged lines
     float* EF = nullptr;    // device: E[N], F[N], RN(1/F)[N]
-    float4* FRS = nullptr;  // device: (F, RN(1/F), s, s*RN(1/F)) per element of 32*ceil(N/32), boundary
-                            // elements (0 and >= N-1) as identities (1, 1, 0, 0)
+    float4* FRS = nullptr;  // device: (F, R, s, L) per element of 32*ceil(N/32), R = RN(1/F) and
+                            // L = RN(1/F - R); boundary elements (0 and >= N-1) as identities (1, 1, 0, 0)
     uint32_t* line_flag = nullptr;  // N*N: x-line (y + z*N) holds uptake
     int* line_list = nullptr;       // flagged lines
     int* line_count = nullptr;      // device: number of flagged lines
@@ -66,7 +66,7 @@ struct Substrate {
     // F equal E[N-2], F[N-2] bit for bit: the LU factors of the constant-coefficient line converge
     // within a few dozen elements, so all groups but the first and the last usually qualify.
     uint32_t uniform_groups = 0;
-    float conv_R = 0.f;     // RN(1/F[N-2]), the reciprocal of the converged F
+    float conv_R = 0.f, conv_L = 0.f;  // the reciprocal of the converged F, F[N-2], as R + L
     CUtensorMap tmap[3];    // TMA maps of the field for the x, y and z sweeps (32x32 boxes)
 };
 

@@ -23,10 +23,14 @@
 // Arithmetic per line, the reference kernels' with nvcc's multiply-add fusion:
 //   Y0 = b; Y_i = fma(-E_i, Y_{i-1}, p_i) (i = 1..N-2); x_{N-1} = b;
 //   x_i = fma(-s, x_{i+1}, Y_i) / F_i (i = N-2..1); x_0 = b;  s = E[1]*F[0]
-// and the source p /= fma(-rate, dt, 1).  The division on the back-substitution chain is
-// Markstein's (IBM J. Res. Dev. 34(1), 1990): with y = RN(1/F_i) precomputed on the host, two
-// residual corrections q += (a - F q) y give the correctly rounded quotient, equal to IEEE
-// division (checked against it by gell_selftest_division and by the bit-exact parity tests).
+// and the source p /= fma(-rate, dt, 1).  The division by F_i on the back-substitution chain uses
+// 1/F_i as an unevaluated sum R + L of two floats precomputed on the host (Brisebarre, Muller, Raina,
+// IEEE Trans. Computers 53(8), 2004): q = fma(t, R, t L) is the correctly rounded t / F_i but for
+// about one quotient in 2^22, and t L, which needs few bits, is taken as fma(-s L, x, Y L) beside
+// t = fma(-s, x, Y), so that the chain from one element to the next is two multiply-adds.  Every q is
+// compared with Markstein's correction of it (IBM J. Res. Dev. 34(1), 1990: q + (t - F q) R is exact
+// from a q this close), and a group where any differs is redone with Markstein's division from t R.
+// Both are checked against IEEE division by gell_selftest_division and the bit-exact parity tests.
 #include <cuda.h>
 
 #include <cstring>
@@ -48,13 +52,12 @@ struct SubDev {
     const float* rate;
     const uint32_t* line_flag;
     const float* EFR;  // E[N], F[N], RN(1/F)[N]
-    const float4* FRS; // per element (F, RN(1/F), s, s*RN(1/F)), boundary elements as identities
+    const float4* FRS; // per element (F, R, s, L), 1/F = R + L; boundary elements as identities
     float b;
     float side;
-    // groups whose E, F are the line's converged constants, and those constants pre-negated:
-    // -E, -s, -s*RN(1/F), -F and RN(1/F)
+    // groups whose E, F are the line's converged constants, and those constants: -E, -s, -s*L, -F, R, L
     uint32_t uni;
-    float nE, nS, nSR, nF, R;
+    float nE, nS, nSL, nF, R, L;
 };
 
 struct LodArgs {
@@ -150,12 +153,12 @@ __device__ __forceinline__ void box_store(const LodArgs& a, const TileDesc& d, i
 }
 
 // Per-element tables.  Boundary elements (j = 0 and j >= N-1) are identities: E = 0 makes
-// Y_j = p_j (= b, set by the pre-pass), and (F, 1/F, s) = (1, 1, 0) makes x_j = Y_j = b, which is
+// Y_j = p_j (= b, set by the pre-pass), and (F, R, s, L) = (1, 1, 0, 0) makes x_j = Y_j = b, which is
 // what the reference's x_0 = x_{N-1} = b gives (it never uses Y at N-1).  Every group therefore
 // runs the same code.
 struct SweepCtx {
     const float* E;    // E[j] (16-byte aligned)
-    const float4* FR;  // (F[j], RN(1/F[j]), s[j], 0) (16-byte aligned)
+    const float4* FR;  // (F[j], R[j], s[j], L[j]) (16-byte aligned)
     float b, dt;
 };
 
@@ -249,9 +252,9 @@ __device__ __forceinline__ float back_exact(float x, float y, float f, float rf,
 }
 
 // Back substitution over a full group (elements 32g+31 .. 32g, all in [1, N-2]), results in o[].
-// The chain carries a1, the once-corrected quotient started from fma(-s/F, x, y/F); the exact
-// quotient a2 is computed beside it.  If any lane's a1 differs from its a2 anywhere in the group,
-// the whole group is recomputed on the exact chain, so o[] always holds the exact values.
+// The chain carries a1 = fma(t, R, t L); the exact quotient a2 is computed beside it.  If any lane's
+// a1 differs from its a2 anywhere in the group, the whole group is recomputed on the exact chain, so
+// o[] always holds the exact values.
 template <int AXIS>
 __device__ __forceinline__ void backward_full(const SweepCtx& c, float* slot, int j0, int lane, float& x,
                                               float o[32], int exact) {
@@ -270,15 +273,16 @@ __device__ __forceinline__ void backward_full(const SweepCtx& c, float* slot, in
 #pragma unroll
             for (int k = 0; k < 8; ++k) h[k] = __ldg(fb + 8 * b8 - 8 + k);
         }
-        float yr[8];
+        float yl[8], sl[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) yr[k] = __fmul_rn(v[k], f[k].y);
+        for (int k = 0; k < 8; ++k) {
+            yl[k] = __fmul_rn(v[k], f[k].w);
+            sl[k] = __fmul_rn(-f[k].z, f[k].w);
+        }
 #pragma unroll
         for (int k = 7; k >= 0; --k) {
             const float t = __fmaf_rn(-f[k].z, x, v[k]);
-            const float a0 = __fmaf_rn(-f[k].w, x, yr[k]);
-            const float r0 = __fmaf_rn(-a0, f[k].x, t);
-            const float a1 = __fmaf_rn(r0, f[k].y, a0);   // carried on the chain
+            const float a1 = __fmaf_rn(t, f[k].y, __fmaf_rn(sl[k], x, yl[k]));  // carried on the chain
             const float r1 = __fmaf_rn(-a1, f[k].x, t);
             const float a2 = __fmaf_rn(r1, f[k].y, a1);   // exact quotient of t by F
             bad |= __float_as_uint(a1) ^ __float_as_uint(a2);
@@ -329,32 +333,34 @@ __device__ __forceinline__ void forward_uniform(float* slot, int g, int lane, fl
     }
 }
 
+// What bounds it is the chain from one element to the next (one warp per scheduler): two dependent
+// operations since the quotient is taken from a reciprocal in two floats, three before (three sweeps of
+// 400^3 x 2 substrates 0.221 / 0.218 / 0.208 ms before, 0.211 / 0.206 / 0.197 after).
 template <int AXIS>
 __device__ __forceinline__ void backward_uniform(const SubDev& sd, float* slot, int lane, float& x, float o[32],
                                                  int exact) {
     const float x_in = x;
     const float R = sd.R, nF = sd.nF;
-    const float2 nS2 = make_float2(sd.nS, sd.nSR), R2 = make_float2(R, R), nF2 = make_float2(nF, nF);
+    const float2 nS2 = make_float2(sd.nS, sd.nSL), L2 = make_float2(sd.L, sd.L), R2 = make_float2(R, R), nF2 = make_float2(nF, nF);
     uint32_t bad = 0;
     float v[8], w[8];
     load8<AXIS>(slot, 24, lane, v);
 #pragma unroll
     for (int b8 = 3; b8 >= 0; --b8) {
         if (b8 > 0) load8<AXIS>(slot, 8 * b8 - 8, lane, w);
-        float yr[8];
+        float yl[8];
 #pragma unroll
         for (int k = 0; k < 8; k += 2) {
-            const float2 q = __fmul2_rn(make_float2(v[k], v[k + 1]), R2);
-            yr[k] = q.x;
-            yr[k + 1] = q.y;
+            const float2 q = __fmul2_rn(make_float2(v[k], v[k + 1]), L2);
+            yl[k] = q.x;
+            yl[k + 1] = q.y;
         }
         float t[8], a1[8];
 #pragma unroll
         for (int k = 7; k >= 0; --k) {
-            // (t, a0) = (fma(-s, x, y), fma(-s/F, x, y/F))
-            const float2 ta = __ffma2_rn(nS2, make_float2(x, x), make_float2(v[k], yr[k]));
-            const float r0 = __fmaf_rn(ta.y, nF, ta.x);
-            x = __fmaf_rn(r0, R, ta.y);  // a1, carried on the chain
+            // (t, t L) = (fma(-s, x, y), fma(-s L, x, y L))
+            const float2 ta = __ffma2_rn(nS2, make_float2(x, x), make_float2(v[k], yl[k]));
+            x = __fmaf_rn(ta.x, R, ta.y);  // a1, carried on the chain
             t[k] = ta.x;
             a1[k] = x;
             o[8 * b8 + k] = x;
@@ -1122,7 +1128,7 @@ __global__ void k_wait_check(int polls, int* err) {
     mbar_wait(&bar, 0u, err, 12, polls);
 }
 
-// Markstein division against IEEE division on random operands in the sweeps' range.
+// The sweeps' two divisions against IEEE division on random operands in the sweeps' range.
 __global__ void k_div_check(long long n, unsigned long long seed, unsigned long long* bad) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -1132,7 +1138,11 @@ __global__ void k_div_check(long long n, unsigned long long seed, unsigned long 
     const float a = __uint_as_float((r.x & 0x80000000u) | ((107u + (r.y % 41u)) << 23) | (r.z & 0x7fffffu));
     const float f = __uint_as_float((127u + (r.w % 6u)) << 23 | (r.x & 0x7fffffu));
     const float y = __frcp_rn(f);
-    if (__float_as_uint(div_rn(a, f, y)) != __float_as_uint(__fdiv_rn(a, f))) atomicAdd(bad, 1ull);
+    const uint32_t e = __float_as_uint(__fdiv_rn(a, f));
+    // the sweeps' quotient (from a reciprocal in two floats) after its correction, and the exact chain's
+    const float q = __fmaf_rn(a, y, __fmul_rn(a, __fmul_rn(__fmaf_rn(-y, f, 1.f), y)));
+    const float c = __fmaf_rn(__fmaf_rn(-q, f, a), y, q);
+    if (__float_as_uint(div_rn(a, f, y)) != e || __float_as_uint(c) != e) atomicAdd(bad, 1ull);
 }
 
 // Setboundary + meshupdatekernel on the x-lines that hold uptake (the lines PreLOD listed), in
@@ -1352,10 +1362,9 @@ static gell_status lod_solver_range(gell_ctx* c, int s0, int s1, int substeps, c
     for (int s = s0; s < s1; ++s, ++ns) {
         const Substrate& S = c->subs[s];
         const int N = c->g.N;
-        const float R = S.conv_R;
         const SubDev sd{S.p,         S.rate,  S.line_flag,       S.EF,         S.FRS, S.s.boundary,
                         S.side,      S.uniform_groups,           -S.E[N - 2],  -S.side,
-                        -(S.side * R), -S.F[N - 2],              R};
+                        -(S.side * S.conv_L), -S.F[N - 2], S.conv_R, S.conv_L};
         ax.sub[ns] = ay.sub[ns] = az.sub[ns] = sd;
         ax.tm[ns] = S.tmap[0];
         ay.tm[ns] = S.tmap[1];
@@ -1451,9 +1460,8 @@ gell_status lod_batch_build(const std::vector<gell_ctx*>& ms, LodBatch** out) {
             BatchItem it;
             std::memset(&it, 0, sizeof(it));
             for (int k = 0; k < 3; ++k) it.tm[k] = S.tmap[k];
-            const float R = S.conv_R;
-            it.sd = SubDev{S.p,    S.rate,           S.line_flag, S.EF,        S.FRS,      S.s.boundary, S.side,
-                           S.uniform_groups, -S.E[N - 2], -S.side, -(S.side * R), -S.F[N - 2], R};
+                it.sd = SubDev{S.p,    S.rate,           S.line_flag, S.EF,        S.FRS,      S.s.boundary, S.side,
+                           S.uniform_groups, -S.E[N - 2], -S.side, -(S.side * S.conv_L), -S.F[N - 2], S.conv_R, S.conv_L};
             it.g = c->g;
             it.B = B;
             it.exact = c->exact_chain ? 1 : 0;
