@@ -376,7 +376,8 @@ static float recip_rn(float f) {
 static float recip_lo(float f, float r) { return (float)((1.0 - (double)r * (double)f) / (double)f); }
 
 // TMA maps of a pitched field: x boxes [32 lines][32 elements] with the 128-byte swizzle over
-// (P, N*N); y boxes [32 elements][32 lines] over (P, N, N); z boxes over (P*N, N).
+// (P, N*N); y boxes [32 elements][32 lines] over (P, N, N); z boxes over (P*N, N); xy-plane boxes
+// [32 y][32 x] over (P, N, N) with the swizzle of the x boxes.
 static gell_status make_tensor_maps(gell_ctx* c, Substrate& sub) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
@@ -402,6 +403,10 @@ static gell_status make_tensor_maps(gell_ctx* c, Substrate& sub) {
     if (r == CUDA_SUCCESS)
         r = encode(&sub.tmap[2], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, sub.p, dz, sz, box2, es,
                    CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    if (r == CUDA_SUCCESS)
+        r = encode(&sub.tmap[3], CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 3, sub.p, dy, sy, box3, es,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return fail(c, GELL_ERR_CUDA, "cuTensorMapEncodeTiled failed (" + std::to_string((int)r) + ")");
     return GELL_OK;

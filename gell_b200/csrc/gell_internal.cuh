@@ -67,7 +67,7 @@ struct Substrate {
     // within a few dozen elements, so all groups but the first and the last usually qualify.
     uint32_t uniform_groups = 0;
     float conv_R = 0.f, conv_L = 0.f;  // the reciprocal of the converged F, F[N-2], as R + L
-    CUtensorMap tmap[3];    // TMA maps of the field for the x, y and z sweeps (32x32 boxes)
+    CUtensorMap tmap[4];    // TMA maps of the field (32x32 boxes) for the x, y and z sweeps and the xy-planes
 };
 
 // Kernel-side view of the geometry.
@@ -128,6 +128,7 @@ struct gell_ctx {
     cudaEvent_t sub_fork = nullptr;
     bool sweeps_configured = false;  // the sweeps' shared-memory attribute is set on this device
     bool ring_configured = false;    // the same for the ring sweeps
+    bool planes_configured = false;  // and for the plane sweeps
 
     // gell_run_mechanics: captured graphs of two mechanics steps and what each was captured for
     // (two entries: an odd number of steps flips the double buffers to the other assignment)

@@ -165,9 +165,13 @@ struct SweepCtx {
 // Address of element e (0..31) of this lane's line in a slot.  x slots are [line][element] with
 // the 128-byte swizzle (16-byte chunk c of row r stored at chunk c ^ (r & 7)); y/z slots are
 // [element][line].
+// kSwzCol addresses a slot of the x layout (swizzled rows) along its rows: element e is row e, the
+// lane a column, as the fused plane kernels need for their second sweep direction.
+constexpr int kSwzCol = 3;
 template <int AXIS>
 __device__ __forceinline__ float* elem(float* slot, int e, int lane) {
     if (AXIS == 0) return slot + lane * 32 + (((e >> 2) ^ (lane & 7)) << 2) + (e & 3);
+    if (AXIS == kSwzCol) return slot + e * 32 + (((lane >> 2) ^ (e & 7)) << 2) + (lane & 3);
     return slot + e * 32 + lane;
 }
 
@@ -181,7 +185,7 @@ __device__ __forceinline__ void load8(float* slot, int e0, int lane, float v[8])
         v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
     } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = slot[(e0 + k) * 32 + lane];
+        for (int k = 0; k < 8; ++k) v[k] = *elem<AXIS>(slot, e0 + k, lane);
     }
 }
 template <int AXIS>
@@ -191,7 +195,7 @@ __device__ __forceinline__ void store8(float* slot, int e0, int lane, const floa
         *reinterpret_cast<float4*>(elem<0>(slot, e0 + 4, lane)) = make_float4(v[4], v[5], v[6], v[7]);
     } else {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) slot[(e0 + k) * 32 + lane] = v[k];
+        for (int k = 0; k < 8; ++k) *elem<AXIS>(slot, e0 + k, lane) = v[k];
     }
 }
 
@@ -562,6 +566,306 @@ __global__ void __launch_bounds__(64 * kMaxComputeWarps, 1) k_sweep(const __grid
         if (!ok) break;
         d = dn;
     }
+}
+
+// ------------------------------------------------------------------ plane sweeps (N <= 224)
+//
+// Two sweeps in one pass over the field: after k_source_lines,
+//   k_plane  a CTA holds one xy-plane in shared memory: boundary, x sweep, y sweep
+//   k_ztile  one 32-line tile of the z sweep per warp
+// each one wave of CTAs (or little more) that request everything at once.  All three start while the
+// kernel before them drains (programmatic stream serialisation): they set up barriers and tables, then
+// wait (griddepcontrol.wait) before they touch the field.
+//
+// A plane is B x B boxes of 32 x 32 floats in the swizzled x layout (row = lane, 16-byte chunks).  The
+// recurrences work on 32 elements in registers at a time, which keeps shared-memory instructions off
+// the dependent chains (one scheduler issues a shared-memory instruction every 4 cycles, whatever its
+// width): values are loaded 4 at a time, and the x results are written transposed into their own box,
+// so that the y sweep reads its columns 4 at a time as well.
+constexpr int kPlaneMaxN = 224;  // 7 x 7 boxes of 4 KB
+
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+struct LineCtx {
+    const float* E;    // shared: E[j], 0 at the line's ends
+    const float4* FR;  // shared: (-F, R, -s, L), identities (-1, 1, 0, 0) at the ends
+    uint32_t uni;      // groups that hold the line's converged factors
+    float b, nE, nS, nSL, nF, R, L;
+    int exact;
+};
+__device__ __forceinline__ LineCtx line_ctx(const LodArgs& a, const SubDev& sd, const float* sE, const float4* sFR) {
+    return LineCtx{sE, sFR, sd.uni, sd.b, sd.nE, sd.nS, sd.nSL, sd.nF, sd.R, sd.L, a.exact};
+}
+__device__ __forceinline__ void stage_tables(const SubDev& sd, float* sE, float4* sFR, int N, int n, int i0, int di) {
+    for (int j = i0; j < n; j += di) {
+        sE[j] = (j >= 1 && j <= N - 2) ? sd.EFR[j] : 0.f;
+        const float4 f = sd.FRS[j];
+        sFR[j] = make_float4(-f.x, f.y, -f.z, f.w);
+    }
+}
+
+// The 32 elements of this lane's row of a box (swizzled chunks), to and from registers.
+__device__ __forceinline__ void row_load(const float* box, int lane, float v[32]) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        const float4 t = *reinterpret_cast<const float4*>(box + lane * 32 + ((q ^ (lane & 7)) << 2));
+        v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
+    }
+}
+__device__ __forceinline__ void row_store(float* box, int lane, const float v[32]) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+        *reinterpret_cast<float4*>(box + lane * 32 + ((q ^ (lane & 7)) << 2)) =
+            make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+}
+
+// Forward elimination of group g in place: v[k] becomes Y of element 32g + k.  n: elements of the
+// group that are in the line (a group that is not whole is not converged either).
+__device__ __forceinline__ void forward32(const LineCtx& c, int g, int n, float* v, float& Y) {
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+        if (4 * q >= n) break;
+        const float4 e = *reinterpret_cast<const float4*>(c.E + 32 * g + 4 * q);
+        v[4 * q] = Y = __fmaf_rn(-e.x, Y, v[4 * q]);
+        v[4 * q + 1] = Y = __fmaf_rn(-e.y, Y, v[4 * q + 1]);
+        v[4 * q + 2] = Y = __fmaf_rn(-e.z, Y, v[4 * q + 2]);
+        v[4 * q + 3] = Y = __fmaf_rn(-e.w, Y, v[4 * q + 3]);
+    }
+}
+
+// Back substitution of group g from its Y values v: out(k, x) for k = 31 .. 0, as the chain goes.
+// Where any lane's quotient is not the exact one the group is redone on the exact chain and its
+// results are written again.  The factors of a group that is not converged are read four elements
+// ahead of their use (a shared load cannot be moved over the results' stores).
+template <class Out>
+__device__ __forceinline__ void backward32(const LineCtx& c, int g, int n, const float* v, float& x, Out out) {
+    const float x_in = x;
+    uint32_t bad = 0;
+    const bool uni = (c.uni >> g) & 1u;
+    if (uni) {
+#pragma unroll
+        for (int k = 31; k >= 0; --k) {
+            const float t = __fmaf_rn(c.nS, x, v[k]);
+            x = __fmaf_rn(t, c.R, __fmaf_rn(c.nSL, x, __fmul_rn(v[k], c.L)));
+            out(k, x);
+            bad |= __float_as_uint(x) ^ __float_as_uint(__fmaf_rn(__fmaf_rn(x, c.nF, t), c.R, x));
+        }
+    } else {
+        float4 f[4], h[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[i] = c.FR[32 * g + 28 + i];
+#pragma unroll
+        for (int q = 7; q >= 0; --q) {
+            if (q > 0) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i) h[i] = c.FR[32 * g + 4 * q - 4 + i];
+            }
+            if (4 * q < n)
+#pragma unroll
+            for (int i = 3; i >= 0; --i) {
+                const int k = 4 * q + i;
+                const float t = __fmaf_rn(f[i].z, x, v[k]);
+                x = __fmaf_rn(t, f[i].y, __fmaf_rn(__fmul_rn(f[i].z, f[i].w), x, __fmul_rn(v[k], f[i].w)));
+                out(k, x);
+                bad |= __float_as_uint(x) ^ __float_as_uint(__fmaf_rn(__fmaf_rn(x, f[i].x, t), f[i].y, x));
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) f[i] = h[i];
+        }
+    }
+    if (__any_sync(FULL, bad != 0) || c.exact) {
+        // rare: a rolled loop over a copy in local memory keeps the kernel small (its hot code has to
+        // stay in the 32 KB instruction cache: beyond it the issue rate drops by more than half)
+        float w[32];
+#pragma unroll
+        for (int k = 0; k < 32; ++k) w[k] = v[k];
+        x = x_in;
+#pragma unroll 1
+        for (int k = (n < 32 ? n : 32) - 1; k >= 0; --k) {
+            const float4 f = c.FR[32 * g + k];
+            x = div_rn(__fmaf_rn(f.z, x, w[k]), -f.x, f.y);
+            out(k, x);
+        }
+    }
+}
+
+// After a wait that gave up: wait (briefly) for the loads still in flight, which must not outlive the
+// CTA's shared memory.
+__device__ __forceinline__ void line_drain(uint64_t* full, int g, int B, int* err) {
+    for (int h = g; h < B; ++h) mbar_wait(full + h, 0u, err, 20, 1 << 16);
+}
+
+// Shared memory of a plane: B x B boxes, FR and E tables, a barrier per box.
+__host__ __device__ inline size_t plane_smem(int B) { return 1024 + (size_t)B * B * (kSlotFloats * 4 + 8) + (size_t)32 * B * 20; }
+
+// (the bound of 320 threads caps the registers so that two CTAs of 5 warps, N <= 160, fit an SM)
+__global__ void __launch_bounds__(320, 1) k_plane(const __grid_constant__ LodArgs a) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    const int N = a.g.N, P = a.g.P;
+    const int B = (N + 31) >> 5;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int s = blockIdx.x / N, z = blockIdx.x - s * N;
+    const SubDev& sd = a.sub[s];
+    const uint32_t base = smem_u32(sm);
+    unsigned char* sm1 = sm + ((1024 - (base & 1023)) & 1023);
+    float* boxes = reinterpret_cast<float*>(sm1);  // box (row block rb, column block cb) at (rb * B + cb) * 1024 floats
+    float4* sFR = reinterpret_cast<float4*>(sm1 + (size_t)B * B * kSlotFloats * 4);
+    float* sE = reinterpret_cast<float*>(sFR + 32 * B);
+    uint64_t* full = reinterpret_cast<uint64_t*>(sE + 32 * B) + warp * B;  // this warp's row block
+    stage_tables(sd, sE, sFR, N, 32 * B, threadIdx.x, blockDim.x);
+    if (lane < B) mbar_init(full + lane, 1u);
+    fence_mbar_init();
+    __syncthreads();
+    grid_dep_launch();
+    grid_dep_wait();
+
+    float* rows = boxes + (size_t)warp * B * kSlotFloats;
+    if (lane == 0)
+        for (int g = 0; g < B; ++g) {
+            mbar_arrive_expect(full + g, kSlotFloats * 4);
+            tma_load_3d(rows + (size_t)g * kSlotFloats, &a.tm[s], 32 * g, 32 * warp, z, full + g);
+        }
+    const LineCtx c = line_ctx(a, sd, sE, sFR);
+
+    // x sweep of rows 32 warp .. + 31, one per lane
+    {
+        const int y = 32 * warp + lane;
+        const bool interior = y >= 2 && y < N - 2 && z >= 2 && z < N - 2;
+        const long long line = y + (long long)z * N;
+        const bool flagged = y < N && sd.line_flag[line] != 0u;
+        const bool shell = __any_sync(FULL, !interior && !flagged);
+        float Y = c.b;
+        float v[32];
+        for (int g = 0; g < B; ++g) {
+            float* box = rows + (size_t)g * kSlotFloats;
+            if (!mbar_wait(full + g, 0u, a.err, 1)) {
+                line_drain(full, g, B, a.err);
+                break;
+            }
+            row_load(box, lane, v);
+            if (g == 0 || 32 * g + 31 > N - 3 || shell) {
+                // Setboundary: the two outer layers, every element of a row of the y/z faces' layers;
+                // a row with uptake has been prepared: only Y_0 = b and x_{N-1} = b remain
+                const int lo = flagged ? 1 : interior ? 2 : N, hi = flagged ? N - 2 : N - 3;
+#pragma unroll
+                for (int k = 0; k < 32; ++k)
+                    if (32 * g + k < lo || 32 * g + k > hi) v[k] = c.b;
+            }
+            forward32(c, g, N - 32 * g, v, Y);
+            row_store(box, lane, v);
+        }
+        float x = c.b;
+        for (int g = B - 1; g >= 0; --g) {
+            float* box = rows + (size_t)g * kSlotFloats;
+            row_load(box, lane, v);
+            __syncwarp();  // every lane has its row: the box takes the results transposed
+            backward32(c, g, N - 32 * g, v, x, [&](int k, float r) { *elem<kSwzCol>(box, k, lane) = r; });
+        }
+    }
+    __syncthreads();
+    // y sweep of columns 32 warp .. + 31, one per lane; the boxes hold [column][row]
+    {
+        const float* cols = boxes + (size_t)warp * kSlotFloats;  // box of row block g at g * B * 1024 floats
+        float Y = c.b;
+        float v[32];
+        for (int g = 0; g < B; ++g) {
+            float* box = const_cast<float*>(cols) + (size_t)g * B * kSlotFloats;
+            row_load(box, lane, v);
+            if (g == 0 || 32 * g + 31 > N - 2) {
+#pragma unroll
+                for (int k = 0; k < 32; ++k)
+                    if (32 * g + k == 0 || 32 * g + k >= N - 1) v[k] = c.b;
+            }
+            forward32(c, g, N - 32 * g, v, Y);
+            row_store(box, lane, v);
+        }
+        float x = c.b;
+        for (int g = B - 1; g >= 0; --g) {
+            float* box = const_cast<float*>(cols) + (size_t)g * B * kSlotFloats;
+            row_load(box, lane, v);
+            __syncwarp();  // every lane has its column: the box takes the results as rows again
+            backward32(c, g, N - 32 * g, v, x, [&](int k, float r) { *elem<kSwzCol>(box, k, lane) = r; });
+            fence_proxy_async();
+            __syncwarp();
+            if (lane == 0) {
+                tma_store_3d(&a.tm[s], 32 * warp, 32 * g, z, box);
+                bulk_commit();
+            }
+        }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    }
+}
+
+// One line tile of the z sweep per warp: lanes are 32 consecutive elements of the (x, y) plane.
+constexpr int kTileWarps = 2;
+__host__ __device__ inline size_t tile_smem(int B) { return 1024 + (size_t)kTileWarps * B * (kSlotFloats * 4 + 32 * 20 + 8); }
+
+__global__ void __launch_bounds__(32 * kTileWarps) k_ztile(const __grid_constant__ LodArgs a) {
+    extern __shared__ __align__(1024) unsigned char sm[];
+    const int N = a.g.N;
+    const int B = (N + 31) >> 5;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t base = smem_u32(sm);
+    unsigned char* sm1 = sm + ((1024 - (base & 1023)) & 1023);
+    float* buf = reinterpret_cast<float*>(sm1) + (size_t)warp * B * kSlotFloats;
+    float4* sFR = reinterpret_cast<float4*>(sm1 + (size_t)kTileWarps * B * kSlotFloats * 4) + warp * 32 * B;
+    float* sE = reinterpret_cast<float*>(sm1 + (size_t)kTileWarps * B * (kSlotFloats * 4 + 32 * 16)) + warp * 32 * B;
+    uint64_t* full = reinterpret_cast<uint64_t*>(sm1 + (size_t)kTileWarps * B * (kSlotFloats * 4 + 32 * 20)) + warp * B;
+    const long long per_sub = (a.g.PN + 31) / 32;
+    const long long t = (long long)blockIdx.x * kTileWarps + warp;
+    const bool active = t < per_sub * a.nsub;
+    const int s = active ? (int)(t / per_sub) : 0;
+    const uint32_t L0 = (uint32_t)((t - s * per_sub) * 32);
+    const SubDev& sd = a.sub[s];
+    if (active) {
+        stage_tables(sd, sE, sFR, N, 32 * B, lane, 32);
+        if (lane < B) mbar_init(full + lane, 1u);
+        fence_mbar_init();
+    }
+    __syncwarp();
+    grid_dep_launch();
+    grid_dep_wait();
+    if (!active) return;
+    if (lane == 0)
+        for (int g = 0; g < B; ++g) {
+            mbar_arrive_expect(full + g, kSlotFloats * 4);
+            tma_load_2d(buf + (size_t)g * kSlotFloats, &a.tm[s], (int)L0, 32 * g, full + g);
+        }
+    const LineCtx c = line_ctx(a, sd, sE, sFR);
+    float Y = c.b;
+    float v[32];
+    for (int g = 0; g < B; ++g) {
+        float* box = buf + (size_t)g * kSlotFloats;
+        if (!mbar_wait(full + g, 0u, a.err, 3)) {
+            line_drain(full, g, B, a.err);
+            return;
+        }
+#pragma unroll
+        for (int k = 0; k < 32; ++k) v[k] = box[k * 32 + lane];
+        if (g == 0 || 32 * g + 31 > N - 2) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k)
+                if (32 * g + k == 0 || 32 * g + k >= N - 1) v[k] = c.b;
+        }
+        forward32(c, g, N - 32 * g, v, Y);
+        __syncwarp();  // every lane has its column: the box takes the Y values as rows
+        row_store(box, lane, v);
+    }
+    float x = c.b;
+    for (int g = B - 1; g >= 0; --g) {
+        float* box = buf + (size_t)g * kSlotFloats;
+        row_load(box, lane, v);
+        __syncwarp();  // every lane has its Y values: the box takes the results as columns again
+        backward32(c, g, N - 32 * g, v, x, [&](int k, float q) { box[k * 32 + lane] = q; });
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) {
+            tma_store_2d(&a.tm[s], (int)L0, 32 * g, box);
+            bulk_commit();
+        }
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
 // ------------------------------------------------------------------ ring sweeps
@@ -1160,6 +1464,8 @@ struct SrcArgs {
 };
 
 __global__ void k_source_lines(SrcArgs a) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int N = a.g.N, P = a.g.P;
     const int lane = threadIdx.x & 31;
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1268,6 +1574,22 @@ gell_status prelod(gell_ctx* c, int sub) {
     return GELL_OK;
 }
 
+static SrcArgs source_args(const gell_ctx* c, int s0, int s1) {
+    SrcArgs sa{};
+    for (int s = s0; s < s1; ++s) {
+        const Substrate& S = c->subs[s];
+        sa.p[sa.nsub] = S.p;
+        sa.rate[sa.nsub] = S.rate;
+        sa.list[sa.nsub] = S.line_list;
+        sa.count[sa.nsub] = S.line_count;
+        sa.b[sa.nsub] = S.s.boundary;
+        sa.nsub++;
+    }
+    sa.g = c->g;
+    sa.dt = c->P.diffusion_dt;
+    return sa;
+}
+
 // The ring sweeps (k_sweep_ring): W warps per CTA, each with R group slots, R as large as shared
 // memory allows (at most kRingMaxSlots, at least 2 unless a line is one group).
 static gell_status lod_solver_ring(gell_ctx* c, const LodArgs& ax, const LodArgs& ay, const LodArgs& az, int s0,
@@ -1318,18 +1640,7 @@ static gell_status lod_solver_ring(gell_ctx* c, const LodArgs& ax, const LodArgs
         return (int)(want < cap ? want : cap);
     };
     const int gx = grid(xt, kx), gy = grid(yt, ky), gz = grid(zt, kz);
-    SrcArgs sa{};
-    for (int s = s0; s < s1; ++s) {
-        const Substrate& S = c->subs[s];
-        sa.p[sa.nsub] = S.p;
-        sa.rate[sa.nsub] = S.rate;
-        sa.list[sa.nsub] = S.line_list;
-        sa.count[sa.nsub] = S.line_count;
-        sa.b[sa.nsub] = S.s.boundary;
-        sa.nsub++;
-    }
-    sa.g = c->g;
-    sa.dt = c->P.diffusion_dt;
+    const SrcArgs sa = source_args(c, s0, s1);
     for (int k = 0; k < substeps; ++k) {
         GELL_KERNEL(c, "k_source_lines", k_source_lines<<<source_ctas(), 256, 0, strm>>>(sa));
         if (hint) {
@@ -1355,28 +1666,76 @@ static bool ring_by_default(const gell_ctx* c, int ns) {
     return (227 * 1024 - fixed) / (B * kSlotFloats * 4) < 4;
 }
 
+// A launch whose CTAs may start while the kernel before it on the stream drains (the kernel itself
+// waits for that kernel's results).
+template <class K, class... A>
+static void launch_dependent(K kern, int grid, int block, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
+// The plane sweeps serve every grid whose plane fits in one CTA's shared memory (N <= 224), unless
+// GELL_OPT_SWEEP_RING asks for another kernel.  Ten substeps against the line tiles (which at these
+// sizes wait on 4 launches a substep and on one tile's latency): 16^3 99 against 223 us, 96^3 235
+// against 305, 131^3 x 2 354 against 556, 160^3 337 against 540, 200^3 603 against 854, 224^3 x 2 1330
+// against 1449.
+static bool planes_by_default(const gell_ctx* c) {
+    return c->g.N <= kPlaneMaxN && c->sweep_ring < 0;
+}
+
+static gell_status lod_solver_planes(gell_ctx* c, const LodArgs& axy, const LodArgs& az, const SrcArgs& sa, int substeps,
+                                     cudaStream_t strm) {
+    const int B = (c->g.N + 31) / 32;
+    if (!c->planes_configured) {
+        for (const void* k : {(const void*)k_plane, (const void*)k_ztile})
+            GELL_CUDA(c, cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+        c->planes_configured = true;
+    }
+    const int planes = c->g.N * az.nsub;
+    const long long zt = (c->g.PN + 31) / 32 * az.nsub;
+    const int gz = (int)((zt + kTileWarps - 1) / kTileWarps);
+    // a warp per line that can hold uptake, at most one wave
+    const int lines = (c->g.N * c->g.N + 7) / 8, gs = lines < source_ctas() ? lines : source_ctas();
+    for (int k = 0; k < substeps; ++k) {
+        GELL_KERNEL(c, "k_source_lines", launch_dependent(k_source_lines, gs, 256, 0, strm, sa));
+        GELL_KERNEL(c, "k_plane_xy", launch_dependent(k_plane, planes, 32 * B, plane_smem(B), strm, axy));
+        GELL_KERNEL(c, "k_sweep_z", launch_dependent(k_ztile, gz, 32 * kTileWarps, tile_smem(B), strm, az));
+    }
+    return GELL_OK;
+}
+
 // LOD substeps of substrates [s0, s1) on stream `strm`.
 static gell_status lod_solver_range(gell_ctx* c, int s0, int s1, int substeps, cudaStream_t strm) {
-    LodArgs ax{}, ay{}, az{};
+    LodArgs ax{}, ay{}, az{}, axy{};
     int ns = 0;
     for (int s = s0; s < s1; ++s, ++ns) {
         const Substrate& S = c->subs[s];
         const int N = c->g.N;
         const SubDev sd{S.p,         S.rate,  S.line_flag,       S.EF,         S.FRS, S.s.boundary,
-                        S.side,      S.uniform_groups,           -S.E[N - 2],  -S.side,
-                        -(S.side * S.conv_L), -S.F[N - 2], S.conv_R, S.conv_L};
-        ax.sub[ns] = ay.sub[ns] = az.sub[ns] = sd;
+                        S.side,      S.uniform_groups,           -S.E[N - 2],  -S.side, -(S.side * S.conv_L), -S.F[N - 2], S.conv_R, S.conv_L};
+        ax.sub[ns] = ay.sub[ns] = az.sub[ns] = axy.sub[ns] = sd;
         ax.tm[ns] = S.tmap[0];
         ay.tm[ns] = S.tmap[1];
         az.tm[ns] = S.tmap[2];
+        axy.tm[ns] = S.tmap[3];
     }
-    for (LodArgs* a : {&ax, &ay, &az}) {
+    for (LodArgs* a : {&ax, &ay, &az, &axy}) {
         a->nsub = ns;
         a->g = c->g;
         a->dt = c->P.diffusion_dt;
         a->err = c->dev_err;
         a->exact = c->exact_chain ? 1 : 0;
     }
+    if (planes_by_default(c)) return lod_solver_planes(c, axy, az, source_args(c, s0, s1), substeps, strm);
     const int N = c->g.N;
     const int B = (N + 31) / 32;
     const int Na = (N + 31) & ~31;
@@ -1414,18 +1773,7 @@ static gell_status lod_solver_range(gell_ctx* c, int s0, int s1, int substeps, c
     };
     const int gx = grid(xt, (const void*)k_sweep<0>), gy = grid(yt, (const void*)k_sweep<1>),
               gz = grid(zt, (const void*)k_sweep<2>);
-    SrcArgs sa{};
-    for (int s = s0; s < s1; ++s) {
-        const Substrate& S = c->subs[s];
-        sa.p[sa.nsub] = S.p;
-        sa.rate[sa.nsub] = S.rate;
-        sa.list[sa.nsub] = S.line_list;
-        sa.count[sa.nsub] = S.line_count;
-        sa.b[sa.nsub] = S.s.boundary;
-        sa.nsub++;
-    }
-    sa.g = c->g;
-    sa.dt = c->P.diffusion_dt;
+    const SrcArgs sa = source_args(c, s0, s1);
     for (int k = 0; k < substeps; ++k) {
         GELL_KERNEL(c, "k_source_lines", k_source_lines<<<source_ctas(), 256, 0, strm>>>(sa));
         GELL_KERNEL(c, "k_sweep_x", k_sweep<0><<<gx, w * 64, smem, strm>>>(ax));
@@ -1566,7 +1914,8 @@ static bool substrate_streams(gell_ctx* c, int s0, int s1) {
 gell_status lod_solver(gell_ctx* c, int sub, int substeps) {
     if (c->subs.empty() || substeps == 0) return GELL_OK;
     const int s0 = sub < 0 ? 0 : sub, s1 = sub < 0 ? (int)c->subs.size() : sub + 1;
-    if (!substrate_streams(c, s0, s1)) return lod_solver_range(c, s0, s1, substeps, c->stream);
+    // the plane sweeps take every substrate's planes in one launch
+    if (planes_by_default(c) || !substrate_streams(c, s0, s1)) return lod_solver_range(c, s0, s1, substeps, c->stream);
     GELL_CUDA(c, cudaEventRecord(c->sub_fork, c->stream));
     for (int s = s0 + 1; s < s1; ++s) GELL_CUDA(c, cudaStreamWaitEvent(c->sub_stream[s], c->sub_fork, 0));
     for (int s = s0; s < s1; ++s) {

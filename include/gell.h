@@ -292,7 +292,8 @@ enum {
  * slots of shared memory per warp; back substitution re-reads each group from L2 and recomputes its
  * forward values from a per-group checkpoint), which fit twice as many warps per SM as whole line
  * tiles; 2..8 do the same with at most that many slots per warp; 0 keeps whole line tiles in shared
- * memory; -1 picks the ring when fewer than four line tiles fit per SM (long lines, N > 416).
+ * memory; -1 picks the plane sweeps (x and y in one pass) where a plane fits in one CTA's shared
+ * memory (N <= 224), else the ring when fewer than four line tiles fit per SM (long lines, N > 416).
  * GELL_OPT_SWEEP_L2HINT (0 or 1, default 0): the ring sweeps load groups they will read again with
  * priority to stay in L2.  GELL_OPT_SWEEP_RING_LAG (0..7, default 0 = 1): how many of its own
  * result stores a ring warp lets run before it refills a stored slot (capped at the slots less
@@ -305,11 +306,12 @@ enum {
  * inputs quantise the change rather than the field.  Weights are trained for one form.
  * GELL_OPT_LOD_STREAMS (0 or 1, default 1): the LOD substeps of each substrate run on a stream of
  * their own (forked from and joined back to the context's stream), so that one substrate's sweep
- * fills the SMs another's leaves idle at its start and end.  Results are identical. */
+ * fills the SMs another's leaves idle at its start and end (the plane sweeps take every substrate in
+ * one launch instead).  Results are identical. */
 /* GELL_OPT_CONV_RING (0 or 1, default 1): the surrogate's convolutions keep the input rows of
  * consecutive lines in a ring of shared-memory slots (each row read from L2 once per unit of 32
  * lines) instead of loading all nine rows per tile; the results are the same. */
-/* GELL_OPT_SWEEP_WARPS (0..4, default 0): line tiles (compute warps) per CTA of the LOD sweeps;
+/* GELL_OPT_SWEEP_WARPS (0..4, default 0): line tiles (compute warps) per CTA of the line-tile sweeps;
  * 0 = as many as shared memory holds.  Fewer give more, smaller CTAs, which can fill the GPU
  * better for small grids run side by side (the ensemble tuner tries them).  Results do not change. */
 gell_status gell_set_option(gell_ctx* ctx, int option, int64_t value);
