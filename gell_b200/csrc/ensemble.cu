@@ -85,7 +85,7 @@ gell_status capture(gell_ensemble* e, int substeps) {
     for (int r = 0; r < rounds && ce == cudaSuccess && st == GELL_OK; ++r) {
         if (mech_batched) {
             st = gell::mech_batch_step(e->m, e->origin);
-            if (st == GELL_OK) st = gell::lod_batch_run(e->batch, e->origin, substeps);
+            if (st == GELL_OK) st = gell::lod_batch_run(e->batch, e->origin, substeps, e->fork, e->pool, e->join);
             continue;
         }
         ce = cudaEventRecord(e->fork, e->origin);
@@ -100,7 +100,7 @@ gell_status capture(gell_ensemble* e, int substeps) {
             ce = cudaEventRecord(e->join[b], e->pool[b]);
             if (ce == cudaSuccess) ce = cudaStreamWaitEvent(e->origin, e->join[b], 0);
         }
-        if (e->batched && ce == cudaSuccess && st == GELL_OK) st = gell::lod_batch_run(e->batch, e->origin, substeps);
+        if (e->batched && ce == cudaSuccess && st == GELL_OK) st = gell::lod_batch_run(e->batch, e->origin, substeps, e->fork, e->pool, e->join);
     }
     cudaGraph_t g = nullptr;
     const cudaError_t ee = cudaStreamEndCapture(e->origin, &g);

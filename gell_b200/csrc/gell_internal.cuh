@@ -277,7 +277,9 @@ gell_status lod_solver(gell_ctx* c, int sub, int substeps);
 // `substeps` substeps of every member on `st`.
 struct LodBatch;
 gell_status lod_batch_build(const std::vector<gell_ctx*>& members, LodBatch** out);
-gell_status lod_batch_run(LodBatch* b, cudaStream_t st, int substeps);
+// (on branches of `st`: the streams of `pool`, forked and joined with the events)
+gell_status lod_batch_run(LodBatch* b, cudaStream_t st, int substeps, cudaEvent_t fork, const std::vector<cudaStream_t>& pool,
+                          const std::vector<cudaEvent_t>& join);
 void lod_batch_free(LodBatch* b);
 gell_status prelod(gell_ctx* c, int sub);
 // FM_update and PreLOD of every member of an ensemble, one launch per kernel for all members, on

@@ -33,6 +33,7 @@
 // Both are checked against IEEE division by gell_selftest_division and the bit-exact parity tests.
 #include <cuda.h>
 
+#include <array>
 #include <cstring>
 #include <vector>
 
@@ -594,8 +595,8 @@ struct LineCtx {
     float b, nE, nS, nSL, nF, R, L;
     int exact;
 };
-__device__ __forceinline__ LineCtx line_ctx(const LodArgs& a, const SubDev& sd, const float* sE, const float4* sFR) {
-    return LineCtx{sE, sFR, sd.uni, sd.b, sd.nE, sd.nS, sd.nSL, sd.nF, sd.R, sd.L, a.exact};
+__device__ __forceinline__ LineCtx line_ctx(const SubDev& sd, int exact, const float* sE, const float4* sFR) {
+    return LineCtx{sE, sFR, sd.uni, sd.b, sd.nE, sd.nS, sd.nSL, sd.nF, sd.R, sd.L, exact};
 }
 __device__ __forceinline__ void stage_tables(const SubDev& sd, float* sE, float4* sFR, int N, int n, int i0, int di) {
     for (int j = i0; j < n; j += di) {
@@ -699,14 +700,12 @@ __device__ __forceinline__ void line_drain(uint64_t* full, int g, int B, int* er
 // Shared memory of a plane: B x B boxes, FR and E tables, a barrier per box.
 __host__ __device__ inline size_t plane_smem(int B) { return 1024 + (size_t)B * B * (kSlotFloats * 4 + 8) + (size_t)32 * B * 20; }
 
-// (the bound of 320 threads caps the registers so that two CTAs of 5 warps, N <= 160, fit an SM)
-__global__ void __launch_bounds__(320, 1) k_plane(const __grid_constant__ LodArgs a) {
+// One xy-plane of one field: `tm` is its map of plane boxes.
+__device__ __forceinline__ void plane_body(const CUtensorMap* tm, const SubDev& sd, const Geom& geo, int z, int exact, int* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
-    const int N = a.g.N, P = a.g.P;
+    const int N = geo.N;
     const int B = (N + 31) >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int s = blockIdx.x / N, z = blockIdx.x - s * N;
-    const SubDev& sd = a.sub[s];
     const uint32_t base = smem_u32(sm);
     unsigned char* sm1 = sm + ((1024 - (base & 1023)) & 1023);
     float* boxes = reinterpret_cast<float*>(sm1);  // box (row block rb, column block cb) at (rb * B + cb) * 1024 floats
@@ -724,9 +723,9 @@ __global__ void __launch_bounds__(320, 1) k_plane(const __grid_constant__ LodArg
     if (lane == 0)
         for (int g = 0; g < B; ++g) {
             mbar_arrive_expect(full + g, kSlotFloats * 4);
-            tma_load_3d(rows + (size_t)g * kSlotFloats, &a.tm[s], 32 * g, 32 * warp, z, full + g);
+            tma_load_3d(rows + (size_t)g * kSlotFloats, tm, 32 * g, 32 * warp, z, full + g);
         }
-    const LineCtx c = line_ctx(a, sd, sE, sFR);
+    const LineCtx c = line_ctx(sd, exact, sE, sFR);
 
     // x sweep of rows 32 warp .. + 31, one per lane
     {
@@ -739,8 +738,8 @@ __global__ void __launch_bounds__(320, 1) k_plane(const __grid_constant__ LodArg
         float v[32];
         for (int g = 0; g < B; ++g) {
             float* box = rows + (size_t)g * kSlotFloats;
-            if (!mbar_wait(full + g, 0u, a.err, 1)) {
-                line_drain(full, g, B, a.err);
+            if (!mbar_wait(full + g, 0u, err, 1)) {
+                line_drain(full, g, B, err);
                 break;
             }
             row_load(box, lane, v);
@@ -789,7 +788,7 @@ __global__ void __launch_bounds__(320, 1) k_plane(const __grid_constant__ LodArg
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) {
-                tma_store_3d(&a.tm[s], 32 * warp, 32 * g, z, box);
+                tma_store_3d(tm, 32 * warp, 32 * g, z, box);
                 bulk_commit();
             }
         }
@@ -797,13 +796,21 @@ __global__ void __launch_bounds__(320, 1) k_plane(const __grid_constant__ LodArg
     }
 }
 
+// (the bound of 320 threads caps the registers so that two CTAs of 5 warps, N <= 160, fit an SM)
+__global__ void __launch_bounds__(320, 1) k_plane(const __grid_constant__ LodArgs a) {
+    const int s = blockIdx.x / a.g.N;
+    plane_body(&a.tm[s], a.sub[s], a.g, blockIdx.x - s * a.g.N, a.exact, a.err);
+}
+
 // One line tile of the z sweep per warp: lanes are 32 consecutive elements of the (x, y) plane.
 constexpr int kTileWarps = 2;
 __host__ __device__ inline size_t tile_smem(int B) { return 1024 + (size_t)kTileWarps * B * (kSlotFloats * 4 + 32 * 20 + 8); }
 
-__global__ void __launch_bounds__(32 * kTileWarps) k_ztile(const __grid_constant__ LodArgs a) {
+// One tile (lanes L0 .. L0 + 31 of the flattened xy-plane) of one field; `tm` is its map of z boxes.
+__device__ __forceinline__ void ztile_body(const CUtensorMap* tm, const SubDev& sd, const Geom& geo, int L0, bool active, int exact,
+                                           int* err) {
     extern __shared__ __align__(1024) unsigned char sm[];
-    const int N = a.g.N;
+    const int N = geo.N;
     const int B = (N + 31) >> 5;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t base = smem_u32(sm);
@@ -812,12 +819,6 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_ztile(const __grid_constant
     float4* sFR = reinterpret_cast<float4*>(sm1 + (size_t)kTileWarps * B * kSlotFloats * 4) + warp * 32 * B;
     float* sE = reinterpret_cast<float*>(sm1 + (size_t)kTileWarps * B * (kSlotFloats * 4 + 32 * 16)) + warp * 32 * B;
     uint64_t* full = reinterpret_cast<uint64_t*>(sm1 + (size_t)kTileWarps * B * (kSlotFloats * 4 + 32 * 20)) + warp * B;
-    const long long per_sub = (a.g.PN + 31) / 32;
-    const long long t = (long long)blockIdx.x * kTileWarps + warp;
-    const bool active = t < per_sub * a.nsub;
-    const int s = active ? (int)(t / per_sub) : 0;
-    const uint32_t L0 = (uint32_t)((t - s * per_sub) * 32);
-    const SubDev& sd = a.sub[s];
     if (active) {
         stage_tables(sd, sE, sFR, N, 32 * B, lane, 32);
         if (lane < B) mbar_init(full + lane, 1u);
@@ -830,15 +831,15 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_ztile(const __grid_constant
     if (lane == 0)
         for (int g = 0; g < B; ++g) {
             mbar_arrive_expect(full + g, kSlotFloats * 4);
-            tma_load_2d(buf + (size_t)g * kSlotFloats, &a.tm[s], (int)L0, 32 * g, full + g);
+            tma_load_2d(buf + (size_t)g * kSlotFloats, tm, L0, 32 * g, full + g);
         }
-    const LineCtx c = line_ctx(a, sd, sE, sFR);
+    const LineCtx c = line_ctx(sd, exact, sE, sFR);
     float Y = c.b;
     float v[32];
     for (int g = 0; g < B; ++g) {
         float* box = buf + (size_t)g * kSlotFloats;
-        if (!mbar_wait(full + g, 0u, a.err, 3)) {
-            line_drain(full, g, B, a.err);
+        if (!mbar_wait(full + g, 0u, err, 3)) {
+            line_drain(full, g, B, err);
             return;
         }
 #pragma unroll
@@ -861,11 +862,62 @@ __global__ void __launch_bounds__(32 * kTileWarps) k_ztile(const __grid_constant
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) {
-            tma_store_2d(&a.tm[s], (int)L0, 32 * g, box);
+            tma_store_2d(tm, L0, 32 * g, box);
             bulk_commit();
         }
     }
     if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(32 * kTileWarps) k_ztile(const __grid_constant__ LodArgs a) {
+    const long long per_sub = (a.g.PN + 31) / 32;
+    const long long t = (long long)blockIdx.x * kTileWarps + (threadIdx.x >> 5);
+    const bool active = t < per_sub * a.nsub;
+    const int s = active ? (int)(t / per_sub) : 0;
+    ztile_body(&a.tm[s], a.sub[s], a.g, (int)(t - s * per_sub) * 32, active, a.exact, a.err);
+}
+
+// The same over the fields of many grids (ensembles): items of the same B (boxes per plane edge, so that
+// one launch shape fits them all), laid end to end.  24 members of 64^3 .. 160^3, two steps of 10
+// substeps: 8.23 ms with k_sweep_batch's line tiles, 5.50 ms with these.
+constexpr int kPlaneItems = 128;
+struct alignas(64) PlaneItem {
+    CUtensorMap xy, z;
+    SubDev sd;
+    Geom g;
+    int exact;
+};
+struct PlaneBatch {
+    const PlaneItem* items;
+    int* err;
+    int n;
+    int plane0[kPlaneItems + 1], ztile0[kPlaneItems + 1];  // first plane and first z tile of each item
+};
+// the item whose range holds i
+__device__ __forceinline__ int plane_item(const int* start, int n, int i) {
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (start[mid] <= i) lo = mid;
+        else hi = mid;
+    }
+    return lo;
+}
+__global__ void __launch_bounds__(320, 1) k_plane_batch(const __grid_constant__ PlaneBatch a) {
+    const int i = plane_item(a.plane0, a.n, blockIdx.x);
+    const PlaneItem& it = a.items[i];
+    const SubDev sd = it.sd;
+    const Geom g = it.g;
+    plane_body(&it.xy, sd, g, blockIdx.x - a.plane0[i], it.exact, a.err);
+}
+__global__ void __launch_bounds__(32 * kTileWarps) k_ztile_batch(const __grid_constant__ PlaneBatch a) {
+    const int t = blockIdx.x * kTileWarps + (threadIdx.x >> 5);
+    const bool active = t < a.ztile0[a.n];
+    const int i = plane_item(a.ztile0, a.n, active ? t : 0);
+    const PlaneItem& it = a.items[i];
+    const SubDev sd = it.sd;
+    const Geom g = it.g;
+    ztile_body(&it.z, sd, g, (t - a.ztile0[i]) * 32, active, it.exact, a.err);
 }
 
 // ------------------------------------------------------------------ ring sweeps
@@ -1374,6 +1426,8 @@ __global__ void __launch_bounds__(64 * kBatchWarps, 1) k_sweep_batch(const __gri
 // a line's item is the last one whose first index is not after it.  A line (N <= 256 here) is one
 // batch of 8 loads per lane.
 __global__ void k_source_lines_batch(const SrcItem* items, int nitems) {
+    grid_dep_launch();
+    grid_dep_wait();
     const int lane = threadIdx.x & 31;
     const long long gw = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nw = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -1792,11 +1846,20 @@ struct LodBatch {
     long long total[3] = {0, 0, 0}, cost[3] = {0, 0, 0};
     int Bmax = 0;
     gell_ctx* c0 = nullptr;  // launches counted and timeouts reported on the first member
+    // where every grid has planes that fit (N <= kPlaneMaxN): the items by B, each group a chain of its own
+    struct Group {
+        PlaneBatch args{};
+        const SrcItem* src = nullptr;
+        int B = 0, gsrc = 0;
+    };
+    std::vector<Group> groups;
+    PlaneItem* d_planes = nullptr;
 };
 
 gell_status lod_batch_build(const std::vector<gell_ctx*>& ms, LodBatch** out) {
     *out = nullptr;
     std::vector<BatchItem> items;
+    std::vector<std::array<CUtensorMap, 2>> maps;  // plane and z boxes
     std::vector<SrcItem> src;
     long long tot[3] = {0, 0, 0}, cost[3] = {0, 0, 0};
     int Bmax = 0;
@@ -1822,12 +1885,43 @@ gell_status lod_batch_build(const std::vector<gell_ctx*>& ms, LodBatch** out) {
                 cost[k] += tiles[k] * (B + 1);
             }
             items.push_back(it);
+            maps.push_back({S.tmap[3], S.tmap[2]});
             src.push_back(SrcItem{S.p, S.rate, S.line_list, S.line_count, S.s.boundary, c->P.diffusion_dt, N, P});
             if (B > Bmax) Bmax = B;
         }
     }
     if (items.empty()) return GELL_ERR_INVALID_ARG;
     LodBatch* b = new LodBatch;
+    std::vector<PlaneItem> planes;
+    if (Bmax <= kPlaneMaxN / 32) {
+        // by B, the members' order within; SrcItems in the same order (they are only read through groups then)
+        std::vector<SrcItem> sorted;
+        for (int B = Bmax; B >= 1; --B)
+            for (size_t i = 0; i < items.size(); ++i) {
+                const BatchItem& it = items[i];
+                if (it.B != B) continue;
+                if (b->groups.empty() || b->groups.back().B != B || b->groups.back().args.n == kPlaneItems) {
+                    b->groups.emplace_back();
+                    b->groups.back().B = B;
+                }
+                LodBatch::Group& g = b->groups.back();
+                PlaneBatch& a = g.args;
+                PlaneItem p;
+                std::memset(&p, 0, sizeof(p));
+                p.xy = maps[i][0];
+                p.z = maps[i][1];
+                p.sd = it.sd;
+                p.g = it.g;
+                p.exact = it.exact;
+                planes.push_back(p);
+                sorted.push_back(src[i]);
+                a.plane0[a.n + 1] = a.plane0[a.n] + it.g.N;
+                a.ztile0[a.n + 1] = a.ztile0[a.n] + (int)((it.g.PN + 31) / 32);
+                ++a.n;
+                g.gsrc += (it.g.N * it.g.N + 7) / 8;
+            }
+        src = sorted;
+    }
     b->nitems = (int)items.size();
     for (int k = 0; k < 3; ++k) {
         b->total[k] = tot[k];
@@ -1839,11 +1933,23 @@ gell_status lod_batch_build(const std::vector<gell_ctx*>& ms, LodBatch** out) {
               cudaMalloc((void**)&b->d_src, sizeof(SrcItem) * src.size()) == cudaSuccess &&
               cudaMemcpy(b->d_items, items.data(), sizeof(BatchItem) * items.size(), cudaMemcpyHostToDevice) == cudaSuccess &&
               cudaMemcpy(b->d_src, src.data(), sizeof(SrcItem) * src.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+    if (ok && !planes.empty()) {
+        ok = cudaMalloc((void**)&b->d_planes, sizeof(PlaneItem) * planes.size()) == cudaSuccess &&
+             cudaMemcpy(b->d_planes, planes.data(), sizeof(PlaneItem) * planes.size(), cudaMemcpyHostToDevice) == cudaSuccess;
+        int first = 0;
+        for (LodBatch::Group& g : b->groups) {
+            g.args.items = b->d_planes + first;
+            g.args.err = ms[0]->dev_err;
+            g.src = b->d_src + first;
+            first += g.args.n;
+        }
+    }
     static bool configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
     if (ok && dev >= 0 && dev < 64 && !configured[dev]) {
-        for (const void* k : {(const void*)k_sweep_batch<0>, (const void*)k_sweep_batch<1>, (const void*)k_sweep_batch<2>})
+        for (const void* k : {(const void*)k_sweep_batch<0>, (const void*)k_sweep_batch<1>, (const void*)k_sweep_batch<2>,
+                              (const void*)k_plane_batch, (const void*)k_ztile_batch})
             ok = ok && cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess;
         configured[dev] = ok;
     }
@@ -1860,11 +1966,41 @@ void lod_batch_free(LodBatch* b) {
     if (!b) return;
     if (b->d_items) cudaFree(b->d_items);
     if (b->d_src) cudaFree(b->d_src);
+    if (b->d_planes) cudaFree(b->d_planes);
     delete b;
 }
 
-gell_status lod_batch_run(LodBatch* b, cudaStream_t st, int substeps) {
+// The plane sweeps' substeps of every group on a branch of its own: their fields are independent, so the
+// groups fill the SMs that another one's launches leave idle.
+static gell_status lod_batch_planes(LodBatch* b, cudaStream_t st, int substeps, cudaEvent_t fork,
+                                    const std::vector<cudaStream_t>& pool, const std::vector<cudaEvent_t>& join) {
     gell_ctx* c = b->c0;
+    const size_t nb = pool.size() < b->groups.size() ? pool.size() : b->groups.size();
+    GELL_CUDA(c, cudaEventRecord(fork, st));
+    for (size_t i = 0; i < nb; ++i) GELL_CUDA(c, cudaStreamWaitEvent(pool[i], fork, 0));
+    for (size_t i = 0; i < b->groups.size(); ++i) {
+        const LodBatch::Group& g = b->groups[i];
+        const PlaneBatch& a = g.args;
+        const cudaStream_t s = pool[i % nb];
+        const int gz = (a.ztile0[a.n] + kTileWarps - 1) / kTileWarps;
+        const int gs = g.gsrc < source_batch_ctas() ? g.gsrc : source_batch_ctas();
+        for (int k = 0; k < substeps; ++k) {
+            GELL_KERNEL(c, "k_source_lines", launch_dependent(k_source_lines_batch, gs, 256, 0, s, g.src, a.n));
+            GELL_KERNEL(c, "k_plane_xy", launch_dependent(k_plane_batch, a.plane0[a.n], 32 * g.B, plane_smem(g.B), s, a));
+            GELL_KERNEL(c, "k_sweep_z", launch_dependent(k_ztile_batch, gz, 32 * kTileWarps, tile_smem(g.B), s, a));
+        }
+    }
+    for (size_t i = 0; i < nb; ++i) {
+        GELL_CUDA(c, cudaEventRecord(join[i], pool[i]));
+        GELL_CUDA(c, cudaStreamWaitEvent(st, join[i], 0));
+    }
+    return GELL_OK;
+}
+
+gell_status lod_batch_run(LodBatch* b, cudaStream_t st, int substeps, cudaEvent_t fork, const std::vector<cudaStream_t>& pool,
+                          const std::vector<cudaEvent_t>& join) {
+    gell_ctx* c = b->c0;
+    if (substeps > 0 && !b->groups.empty()) return lod_batch_planes(b, st, substeps, fork, pool, join);
     const int W = kBatchWarps;
     const int Namax = 32 * b->Bmax;
     const int smem = 1024 + W * b->Bmax * kSlotFloats * 4 + align128(W * Namax * 4) + 2 * W * kBatchMaxGroups * 8;

@@ -367,8 +367,10 @@ gell_status gell_reference_spheroid(const gell_params* p, int n, float cell_radi
  * gell_ensemble_set_batched (0 or 1, default 0): every captured step runs the FM_update and PreLOD
  * of ALL members as one launch per kernel (keys, each radix-sort pass, gather, force and move,
  * uptake map; up to 64 members with up to 4 substrates each, larger ensembles run these on the
- * branches), then their LOD substeps as one launch per sweep axis (and one for the uptake source)
- * over a device-side list of every member's line tiles; grid edges up to 256.  Results are
+ * branches), then their LOD substeps: with grid edges up to 224 the plane sweeps, the members of
+ * equal boxes per edge (N / 32 rounded up) in one launch and each such group a branch of its own;
+ * else one launch per sweep axis (and one for the uptake source) over a device-side list of every
+ * member's line tiles, edges up to 256.  Results are
  * identical either way.  gell_ensemble_get_batched reports the setting (after a tune, whether the
  * tuner chose it).
  */

@@ -47,3 +47,32 @@ def test_plane_sweeps_bit_exact(N):
         E, F = ol.mesh_init(N, 10.0, s.diffusion, s.decay, 0.01)
         want = ol.lod_substeps(f, rate, E, F, N, 0.01, s.boundary, 3)
         np.testing.assert_array_equal(a, np.asarray(want, np.float32).reshape(-1).view(np.uint32))
+
+
+def test_batched_planes_of_many_members():
+    """More members of one edge than one batched launch takes, and a member of another edge."""
+    edges = [8] * 130 + [40]
+
+    def members():
+        out = []
+        for i, N in enumerate(edges):
+            sim = gb.Simulation(voxel_num=N, voxel_length=10.0, max_cell_num=64, rng_mode=gb.GELL_RNG_PHILOX)
+            sim.add_substrate(gb.oxygen())
+            sim.set_field(0, random_field(N, seed=i))
+            sim.import_cells(one_per_voxel(N, 10.0, seed=i, lo=2, hi=4))
+            out.append(sim)
+        return out
+
+    alone, together = members(), members()
+    for m in alone:
+        for _ in range(3):
+            m.mechanics_step(2)
+    with gb.Ensemble(together) as ens:
+        ens.set_batched(True)
+        ens.configure(branches=4)
+        ens.run_mechanics(3, 2)
+        ens.sync()
+    for a, b in zip(alone, together):
+        np.testing.assert_array_equal(a.field(0).view(np.uint32), b.field(0).view(np.uint32))
+        a.close()
+        b.close()
