@@ -409,7 +409,7 @@ class Simulation:
         self._check(self.lib.gell_set_option(self.h, 6, int(bool(on))), "gell_set_option")
 
     def set_conv_ring(self, on: bool = True) -> None:
-        """The surrogate's convolutions with (default) or without the row ring along y."""
+        """Accepted and without effect: the surrogate's convolutions have one form."""
         self._check(self.lib.gell_set_option(self.h, 4, int(bool(on))), "gell_set_option")
 
     def launch_count(self) -> int:

@@ -764,7 +764,7 @@ gell_status gell_set_option(gell_ctx* c, int option, int64_t value) {
             if (value < 0 || value > 4) return fail(c, GELL_ERR_INVALID_ARG, "sweep warps outside 0..4");
             c->sweep_warps = (int)value;
             return GELL_OK;
-        case GELL_OPT_CONV_RING: c->conv_ring = value != 0; return GELL_OK;
+        case GELL_OPT_CONV_RING: return GELL_OK;
         case GELL_OPT_SWEEP_RING:
             if (value < -1 || value > 8) return fail(c, GELL_ERR_INVALID_ARG, "sweep ring outside -1..8");
             c->sweep_ring = (int)value;

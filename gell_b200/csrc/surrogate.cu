@@ -13,15 +13,8 @@
 // C/8 planes; plane q holds channels 8q..8q+7 of voxel v = x + N*(y + N*z) as 16 contiguous bytes at
 // byte 16*v.  An x-run of voxels of one plane is then exactly the canonical no-swizzle K-major
 // operand layout of the tensor cores (8 rows of 16 bytes per core matrix, consecutive voxels 16
-// bytes apart), so the operand of tap dx is the run staged for dx = 0 moved by 16*dx bytes.
-//
-// k_conv3 (implicit GEMM on tcgen05).  A tile is 128 consecutive voxels of one x-line (M = 128) by
-// all output channels (N = NOUT); K runs over the 27 taps x the input channels, 16 channels per
-// MMA.  Per tile one TMA box per (dy, dz) brings the 130-voxel run x0-1 .. x0+128 of all input
-// planes (zero fill outside the grid gives the padding), 9 boxes in all; the weights of the whole
-// layer stay in shared memory.  Warp 0 issues the TMA loads (two tile stages), one thread of warp 1
-// issues the MMAs into one of two TMEM accumulators and commits them to mbarriers, warps 2-5 read
-// the finished accumulator (tcgen05.ld), apply bias, ReLU / residual / field update and store.
+// bytes apart), so the operand of tap dx is the run staged for dx = 0 moved by 16*dx bytes; zero fill
+// outside the grid gives the padding.
 // Every wait is bounded (codes 21-27 in the context's error word).
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -40,9 +33,8 @@ struct SurrogateState;
 
 namespace {
 
-constexpr int kTileM = 128;                  // voxels per tile
-constexpr int kRunVox = kTileM + 2;          // staged voxels per (dy, dz) run, with the x halo
-constexpr int kRunPlaneB = kRunVox * 16;     // bytes of one plane of one staged run (2080)
+constexpr int kTileM = 128;               // voxels per tile
+constexpr int kRunPlaneB = kTileM * 16;   // bytes of one plane of one staged run of voxels (2048)
 constexpr int kLayers = 10;                  // conv_in, 4 x (conv_a, conv_b), conv_out
 constexpr int kHidden = 32;
 constexpr int kInCh = 3;
@@ -52,8 +44,13 @@ constexpr int kInCh = 3;
 // with aux = the ReLU's stored output; kResMask: residual add, then times [aux > 0]).
 enum ConvMode { kRelu = 0, kResidual = 1, kField = 2, kLinear = 3, kMask = 4, kResMask = 5 };
 
+// Maps of a planes tensor (plane_map) over half voxels, planes in the last dimension: boxes of 128 voxels of
+// one x-line of one plane, of 2 voxels of one plane, and of 128 voxels of all planes.
+struct PlaneMaps {
+    CUtensorMap run, tail, all;
+};
 struct ConvArgs {
-    CUtensorMap in;                 // 5-D map {8, N, N, N, planes}, box {8, 130, 1, 1, planes}
+    PlaneMaps in;
     const uint8_t* w;               // packed weights, the shared-memory image
     const float* bias;              // NOUT
     uint4* out;                     // planes (kRelu, kResidual)
@@ -64,8 +61,7 @@ struct ConvArgs {
     int N, P;
     long long PN;
     long long nvox;                 // N^3: plane length in voxels
-    int tiles_x;
-    long long tiles;
+    int tiles_x, unit_z;
     float scale, bval;              // kField: out = in + scale * d inside, bval on the shell
     int* err;
 };
@@ -106,6 +102,23 @@ __device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uin
         "l"(a), "l"(b), "r"(idesc), "r"(acc)
         : "memory");
 }
+// The same, issued by the lanes with `on` set of a warp that runs the whole loop together: operands that
+// are uniform over the warp then stay in uniform registers, where the instruction wants them.  (From
+// inside a one-lane branch each operand is moved there again: 75 cycles an MMA.)
+__device__ __forceinline__ void mma_bf16_on(uint32_t on, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "setp.ne.b32 q, %5, 0;\n\t"
+        "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc), "r"(on)
+        : "memory");
+}
+__device__ __forceinline__ uint32_t elect_one() {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(r));
+    return r;
+}
 // The mbarrier completes one phase when every MMA issued so far by this thread has finished.
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
@@ -113,7 +126,7 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
-// 32 lanes x 32 columns (x32) or 16 columns (x16) of fp32: thread t gets lane (base lane + t).
+// 32 lanes x 32 columns of fp32: thread t gets lane (base lane + t).
 __device__ __forceinline__ void tmem_ld32(uint32_t a, uint32_t (&v)[32]) {
     asm volatile(
         "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
@@ -124,20 +137,12 @@ __device__ __forceinline__ void tmem_ld32(uint32_t a, uint32_t (&v)[32]) {
           "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
         : "r"(a));
 }
-__device__ __forceinline__ void tmem_ld16(uint32_t a, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(a));
-}
 
-__device__ __forceinline__ void tma_load_5d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, int c3, int c4,
-                                            uint64_t* bar) {
+__device__ __forceinline__ void tma_load_4d(void* dst, const CUtensorMap* tm, int c0, int c1, int c2, int c3, uint64_t* bar) {
     asm volatile(
-        "cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, "
-        "%6}], [%7];" ::"r"(smem_u32(dst)),
-        "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(smem_u32(bar))
+        "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+        "[%6];" ::"r"(smem_u32(dst)),
+        "l"(tm), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
         : "memory");
 }
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -156,38 +161,35 @@ __device__ __forceinline__ float2 unpack_bf16(uint32_t u) {
     return __bfloat1622float2(h);
 }
 
-// Shared memory of one k_conv3 instance: two tile stages of 9 runs (each run padded to 128 bytes),
-// the layer's weights, ten mbarriers and the TMEM address.
-template <int CIN8, int NOUT>
-struct ConvSmem {
-    static constexpr int kRunB = (CIN8 * kRunPlaneB + 127) / 128 * 128;
-    static constexpr int kStageB = 9 * kRunB;
-    static constexpr int kHalves = CIN8 / 2;               // MMAs (16 input channels) per tap
-    static constexpr int kWBlk = NOUT * 32;                // one (tap, half) weight block
-    static constexpr int kWB = 27 * kHalves * kWBlk;
-    static constexpr int kBars = 2 * kStageB + kWB;
-    static constexpr int kBytes = kBars + 10 * 8 + 16;
+// What the epilogue of one accumulator row (voxel x of line (y, z)) reads besides the accumulator.
+template <int NOUT, int MODE>
+struct TileIn {
+    static constexpr bool kRes = MODE == kResidual || MODE == kResMask, kAux = MODE == kMask || MODE == kResMask;
+    uint4 res[kRes ? NOUT / 8 : 1], aux[kAux ? NOUT / 8 : 1];
+    float field;
+    __device__ __forceinline__ void request(const ConvArgs& a, int x, int y, int z) {
+        if (x >= a.N) return;
+        const long long vox = (long long)x + (long long)a.N * (y + (long long)a.N * z);
+#pragma unroll
+        for (int pl = 0; pl < NOUT / 8; ++pl) {
+            if constexpr (kRes) res[pl] = a.res[pl * a.nvox + vox];
+            if constexpr (kAux) aux[pl] = a.aux[pl * a.nvox + vox];
+        }
+        if constexpr (MODE == kField) field = a.field_in[(long long)x + (long long)a.P * y + a.PN * z];
+    }
 };
 
-__device__ __forceinline__ void tile_of(const ConvArgs& a, long long t, int& x0, int& y, int& z) {
-    const long long line = t / a.tiles_x;
-    x0 = (int)(t - line * a.tiles_x) * kTileM;
-    y = (int)(line % a.N);
-    z = (int)(line / a.N);
-}
-
-// Epilogue of one accumulator row (voxel x of line (y, z)): bias, then ReLU, residual add or the
-// field update, and the store.
+// Epilogue of one accumulator row: bias, then ReLU, residual add or the field update, and the store.
 template <int NOUT, int MODE>
 __device__ __forceinline__ void store_tile(const ConvArgs& a, const uint32_t (&v)[NOUT], const float (&bias)[NOUT],
-                                           int x, int y, int z) {
+                                           const TileIn<NOUT, MODE>& in, int x, int y, int z) {
     if (x >= a.N) return;
     if constexpr (MODE == kField) {
         const long long pi = (long long)x + (long long)a.P * y + a.PN * z;
         const int N = a.N;
         const bool shell = x < 2 || x > N - 3 || y < 2 || y > N - 3 || z < 2 || z > N - 3;
         const float d = __uint_as_float(v[0]) + bias[0];
-        a.field_out[pi] = shell ? a.bval : __fmaf_rn(a.scale, d, a.field_in[pi]);
+        a.field_out[pi] = shell ? a.bval : __fmaf_rn(a.scale, d, in.field);
     } else {
         const long long vox = (long long)x + (long long)a.N * (y + (long long)a.N * z);
         float f[NOUT];
@@ -196,8 +198,7 @@ __device__ __forceinline__ void store_tile(const ConvArgs& a, const uint32_t (&v
 #pragma unroll
         for (int pl = 0; pl < NOUT / 8; ++pl) {
             if constexpr (MODE == kResidual || MODE == kResMask) {
-                const uint4 r = a.res[pl * a.nvox + vox];
-                const uint32_t rr[4] = {r.x, r.y, r.z, r.w};
+                const uint32_t rr[4] = {in.res[pl].x, in.res[pl].y, in.res[pl].z, in.res[pl].w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 u = unpack_bf16(rr[j]);
@@ -206,8 +207,7 @@ __device__ __forceinline__ void store_tile(const ConvArgs& a, const uint32_t (&v
                 }
             }
             if constexpr (MODE == kMask || MODE == kResMask) {
-                const uint4 m = a.aux[pl * a.nvox + vox];
-                const uint32_t mm[4] = {m.x, m.y, m.z, m.w};
+                const uint32_t mm[4] = {in.aux[pl].x, in.aux[pl].y, in.aux[pl].z, in.aux[pl].w};
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float2 u = unpack_bf16(mm[j]);
@@ -226,172 +226,78 @@ __device__ __forceinline__ void store_tile(const ConvArgs& a, const uint32_t (&v
     }
 }
 
-template <int CIN8, int NOUT, int MODE>
-__global__ void __launch_bounds__(192, 1) k_conv3(const __grid_constant__ ConvArgs a) {
-    using L = ConvSmem<CIN8, NOUT>;
-    extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* wsm = smem + 2 * L::kStageB;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
-    uint64_t* full = bars;       // [2] stage loaded
-    uint64_t* empty = bars + 2;  // [2] stage consumed by the MMAs
-    uint64_t* accf = bars + 4;   // [2] accumulator complete
-    uint64_t* acce = bars + 6;   // [2] accumulator read by the epilogue (4 warps)
-    uint64_t* wbar = bars + 8;   // weights loaded
-    uint64_t* done = bars + 9;   // every MMA of this CTA finished
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 10);
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-
-    if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i) {
-            mbar_init(&full[i], 1);
-            mbar_init(&empty[i], 1);
-            mbar_init(&accf[i], 1);
-            mbar_init(&acce[i], 4);
-        }
-        mbar_init(wbar, 1);
-        mbar_init(done, 1);
-        fence_mbar_init();
-    }
-    if (warp == 1) tmem_alloc(tslot, 64);
-    tc_fence_before();
-    __syncthreads();
-    tc_fence_after();
-    const uint32_t tmem = *tslot;
-    const long long T = a.tiles;
-
-    if (warp == 0) {
-        if (lane == 0) {
-            mbar_arrive_expect(wbar, (uint32_t)L::kWB);
-            for (int off = 0; off < L::kWB; off += 16384) {
-                const int nb = L::kWB - off < 16384 ? L::kWB - off : 16384;
-                bulk_load(wsm + off, a.w + off, (uint32_t)nb, wbar);
-            }
-            int k = 0;
-            for (long long t = blockIdx.x; t < T; t += gridDim.x, ++k) {
-                const int s = k & 1;
-                if (k >= 2 && !mbar_wait1(&empty[s], ((k >> 1) - 1) & 1, a.err, 21)) break;
-                int x0, y, z;
-                tile_of(a, t, x0, y, z);
-                uint8_t* st = smem + s * L::kStageB;
-                mbar_arrive_expect(&full[s], (uint32_t)(9 * CIN8 * kRunPlaneB));
-                for (int r = 0; r < 9; ++r)
-                    tma_load_5d(st + r * L::kRunB, &a.in, 0, x0 - 1, y + r % 3 - 1, z + r / 3 - 1, 0, &full[s]);
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = idesc_bf16(NOUT);
-            bool ok = mbar_wait1(wbar, 0, a.err, 22);
-            const uint64_t b0 = sdesc(smem_u32(wsm), NOUT * 16, 128);
-            int k = 0;
-            for (long long t = blockIdx.x; ok && t < T; t += gridDim.x, ++k) {
-                const int s = k & 1;
-                if (!mbar_wait1(&full[s], (k >> 1) & 1, a.err, 23)) break;
-                if (k >= 2 && !mbar_wait1(&acce[s], ((k >> 1) - 1) & 1, a.err, 24)) break;
-                tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(s * 32);
-                const uint64_t a0 = sdesc(smem_u32(smem + s * L::kStageB), kRunPlaneB, 128);
-                // descriptors differ only in the start address (low 14 bits, 16-byte units, no carry
-                // out: shared memory is below 256 KB), so each MMA adds a compile-time offset
-#pragma unroll
-                for (int tap = 0; tap < 27; ++tap) {
-#pragma unroll
-                    for (int h = 0; h < L::kHalves; ++h) {
-                        const uint32_t ao = ((tap / 3) * L::kRunB + (tap % 3) * 16 + 2 * h * kRunPlaneB) >> 4;
-                        const uint32_t bo = ((tap * L::kHalves + h) * L::kWBlk) >> 4;
-                        mma_bf16(d, a0 + ao, b0 + bo, idesc, (tap | h) != 0 ? 1u : 0u);
-                    }
-                }
-                mma_commit(&empty[s]);
-                mma_commit(&accf[s]);
-            }
-            mma_commit(done);
-            mbar_wait1(done, 0, a.err, 25);
-        }
-    } else {
-        const int q = warp & 3;  // TMEM lanes 32q..32q+31 are this warp's
-        float bias[NOUT];
-#pragma unroll
-        for (int n = 0; n < NOUT; ++n) bias[n] = a.bias[n];
-        int k = 0;
-        for (long long t = blockIdx.x; t < T; t += gridDim.x, ++k) {
-            const int s = k & 1;
-            if (!mbar_wait(&accf[s], (k >> 1) & 1, a.err, 26)) break;
-            tc_fence_after();
-            uint32_t v[NOUT];
-            const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(s * 32);
-            if constexpr (NOUT == 32) tmem_ld32(ta, v);
-            else tmem_ld16(ta, v);
-            tmem_wait_ld();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acce[s]);
-            int x0, y, z;
-            tile_of(a, t, x0, y, z);
-            store_tile<NOUT, MODE>(a, v, bias, x0 + 32 * q + lane, y, z);
-        }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (warp == 1) {
-        __syncwarp();
-        tc_fence_after();
-        tmem_dealloc(tmem, 64);
-    }
-}
-
-// ---------------------------------------------------------------- k_conv3_ring
-// The same convolution with the input rows reused along y.  Work comes in units of up to kUnitY
-// consecutive lines y0..y1-1 at one (x tile, z); a unit needs the row groups y0-1 .. y1 (a group =
-// the three runs z-1, z, z+1 at one y, all planes), each loaded once into a ring of kRing group
-// slots and used by the (up to) three tiles y-1, y, y+1 whose taps reach it.  A group's slot is
-// released (tcgen05.commit on its empty barrier) by the last tile that reads it: the oldest group
-// of every tile but the unit's last, and all three groups of the last.  L2 -> shared traffic is
-// one group (3 runs) per tile instead of three.
-constexpr int kUnitY = 32;
+// ---------------------------------------------------------------- k_conv3
+// The 3x3x3 convolution as an implicit GEMM on tcgen05.  A tile is 128 voxels of one x-line (M = 128) by
+// the output channels; K is 27 taps x the input channels, 16 to an MMA.  An MMA's cost is the fetch of its
+// 4 KB A operand from shared memory, whatever its width, so the three z taps of an input line are three
+// column groups of one MMA (N = 3 NOUT): line z' adds to the accumulators of the output lines z'-1, z',
+// z'+1, which lie side by side in tensor memory, and every input line is multiplied by 18 MMAs (32
+// channels) instead of taking part in 54.  (27 separate taps of N = NOUT: 69 cycles an MMA, 3,700 of a
+// tile's 5,200 cycles.)  Each output still is one accumulator's sum over the taps in the order dz, dy, dx.
+//
+// Work comes in units: up to kUnitZ consecutive output lines z0 .. z1-1 at one x tile and y; accumulator i
+// is line z0 + i.  The input lines z0-1 .. z1 pass through a ring of kRing slots: the runs y-1, y, y+1 of
+// 130 voxels, each plane at a multiple of 128 bytes, so that the taps dx = 0 read whole core matrices (the
+// other two straddle them, which doubles the fetch).  A run's plane comes as one box of 128 voxels and one
+// of the last two: rows of 2 KB, since boxes of 16-byte rows (8 channels of a voxel) cost the TMA unit two
+// cycles a row.  Warp 0 issues the MMAs, warps 1-3 the loads (one dy each), and two groups of four
+// epilogue warps take the lines of even and odd index.
+//
+// (256^3, 32 -> 32 channels: 2.52 -> 0.90 ms a launch; what bounds it now is shared memory: 77 cycles of
+// operand fetch an MMA and the staging's writes, 1,600 of a line's 1,700 cycles.)
+constexpr int kUnitZ = 16;    // accumulators: 16 x 32 columns are all of tensor memory
 constexpr int kRing = 6;
+constexpr int kPlaneB = 2176; // bytes from one plane of a staged run to the next: 130 voxels, rounded up to 128 bytes
+constexpr int kConvThreads = 384;
 
 template <int CIN8, int NOUT>
-struct RingSmem {
-    static constexpr int kRunB = (CIN8 * kRunPlaneB + 127) / 128 * 128;
+struct ConvSmem {
+    static constexpr int kRunB = CIN8 * kPlaneB;
     static constexpr int kGroupB = 3 * kRunB;
-    static constexpr int kHalves = CIN8 / 2;
-    static constexpr int kWBlk = NOUT * 32;
-    static constexpr int kWB = 27 * kHalves * kWBlk;
+    static constexpr int kHalves = CIN8 / 2;               // MMAs (16 input channels) per (dy, dx)
+    static constexpr int kWBlk = 3 * NOUT * 32;            // one (dy, dx, half) weight block
+    static constexpr int kWB = 9 * kHalves * kWBlk;
     static constexpr int kBars = kRing * kGroupB + kWB;
-    static constexpr int kBytes = kBars + (2 * kRing + 6) * 8 + 16;
+    static constexpr int kBytes = kBars + (2 * kRing + 2 * kUnitZ + 2) * 8 + 16;
 };
 
-__device__ __forceinline__ void unit_of(const ConvArgs& a, long long u, int& x0, int& y0, int& y1, int& z) {
-    const int nyc = (a.N + kUnitY - 1) / kUnitY;
-    const long long r = u / a.tiles_x;
-    x0 = (int)(u - r * a.tiles_x) * kTileM;
-    y0 = (int)(r % nyc) * kUnitY;
-    y1 = y0 + kUnitY < a.N ? y0 + kUnitY : a.N;
-    z = (int)(r / nyc);
+struct Unit {
+    int x0, y, z0, z1;
+};
+__device__ __forceinline__ Unit unit_of(int N, int tiles_x, int unit_z, long long u) {
+    const long long r = u / tiles_x, s = r / N;
+    Unit o;
+    o.x0 = (int)(u - r * tiles_x) * kTileM;
+    o.y = (int)(r - s * N);
+    o.z0 = (int)s * unit_z;
+    o.z1 = o.z0 + unit_z < N ? o.z0 + unit_z : N;
+    return o;
+}
+__device__ __forceinline__ long long unit_count(int N, int tiles_x, int unit_z) {
+    return (long long)tiles_x * ((N + unit_z - 1) / unit_z) * N;
 }
 
 template <int CIN8, int NOUT, int MODE>
-__global__ void __launch_bounds__(192, 1) k_conv3_ring(const __grid_constant__ ConvArgs a) {
-    using L = RingSmem<CIN8, NOUT>;
+__global__ void __launch_bounds__(kConvThreads, 1) k_conv3(const __grid_constant__ ConvArgs a) {
+    using L = ConvSmem<CIN8, NOUT>;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* wsm = smem + kRing * L::kGroupB;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
-    uint64_t* full = bars;               // [kRing] group loaded
-    uint64_t* empty = bars + kRing;      // [kRing] group released by the MMAs
-    uint64_t* accf = bars + 2 * kRing;   // [2]
-    uint64_t* acce = accf + 2;           // [2] (4 epilogue warps)
-    uint64_t* wbar = acce + 2;
+    uint64_t* full = bars;               // [kRing] input line loaded (three producers)
+    uint64_t* empty = bars + kRing;      // [kRing] input line released by the MMAs
+    uint64_t* accf = bars + 2 * kRing;   // [kUnitZ] accumulator complete
+    uint64_t* acce = accf + kUnitZ;      // [kUnitZ] accumulator read (4 epilogue warps)
+    uint64_t* wbar = acce + kUnitZ;
     uint64_t* done = wbar + 1;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < kRing; ++i) {
-            mbar_init(&full[i], 1);
+            mbar_init(&full[i], 3);
             mbar_init(&empty[i], 1);
         }
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kUnitZ; ++i) {
             mbar_init(&accf[i], 1);
             mbar_init(&acce[i], 4);
         }
@@ -399,168 +305,213 @@ __global__ void __launch_bounds__(192, 1) k_conv3_ring(const __grid_constant__ C
         mbar_init(done, 1);
         fence_mbar_init();
     }
-    if (warp == 1) tmem_alloc(tslot, 64);
+    if (warp == 0) tmem_alloc(tslot, 512);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
-    const int nyc = (a.N + kUnitY - 1) / kUnitY;
-    const long long U = (long long)a.tiles_x * nyc * a.N;
+    const long long U = unit_count(a.N, a.tiles_x, a.unit_z);
 
     if (warp == 0) {
+        // the whole warp runs the loop, one lane issues (see mma_bf16_on)
+        const uint32_t on = elect_one();
+        bool ok = mbar_wait(wbar, 0, a.err, 22);
+        const uint64_t b0 = sdesc(smem_u32(wsm), 3 * NOUT * 16, 128);
+        const uint32_t rbase = smem_u32(smem);
+        uint32_t used = 0, phase = 0;  // per accumulator: written before; parity of its last hand-over
+        auto wait_acc = [&](int m, int nz) {  // an output line's accumulator has been read before line m starts it
+            if (m >= nz) return true;
+            const uint32_t bit = 1u << m;
+            if (used & bit) {
+                if (!mbar_wait(&acce[m], (phase & bit) != 0u, a.err, 24)) return false;
+                phase ^= bit;
+            }
+            used |= bit;
+            return true;
+        };
+        long long u = blockIdx.x;
+        int m = 0, nz = 0, sl = 0;  // input line z0 - 1 + m of the unit, in ring slot sl
+        uint32_t gph = 0;           // parity of the ring's current round
+        // the hand-overs of the line before (its slot; the output line it completed): they are committed a
+        // few MMAs into this line, because the warp cannot go on from a commit before the tensor pipe has
+        // drained up to it, and the pipe then has these MMAs to run through the next commits and waits
+        int csl = -1, cacc = -1;
+        auto commit = [&] {
+            if (on && csl >= 0) {
+                mma_commit(&empty[csl]);
+                if (cacc >= 0) mma_commit(&accf[cacc]);
+            }
+            __syncwarp();
+        };
+        if (u < U) {
+            const Unit w = unit_of(a.N, a.tiles_x, a.unit_z, u);
+            nz = w.z1 - w.z0;
+        }
+        while (ok && u < U) {
+            ok = mbar_wait(&full[sl], gph, a.err, 23);
+            if (ok) ok = wait_acc(m, nz);
+            if (!ok) break;
+            tc_fence_after();
+            // output lines lo .. hi: m-2 (dz = 2), m-1 (dz = 1), m (dz = 0), as far as the unit has them
+            const int lo = m > 2 ? m - 2 : 0, hi = m < nz ? m : nz - 1, n = hi - lo + 1;
+            const bool first = hi == m;  // line m starts here
+            const uint32_t d = tmem + (uint32_t)(lo * NOUT), dm = tmem + (uint32_t)(m * NOUT);
+            const uint64_t bl = b0 + (uint64_t)((lo - m + 2) * NOUT);  // rows of 16 bytes
+            const uint64_t ga = sdesc(rbase + (uint32_t)(sl * L::kGroupB), kPlaneB, 128);
+            const uint32_t idn = idesc_bf16(NOUT * n);
+            // descriptors differ only in the start address (low 14 bits, 16-byte units, no carry out:
+            // shared memory is below 256 KB).  The line's first sum starts from zero, the others' go on.
+            if (first) {
+                if (n > 1) mma_bf16_on(on, d, ga, bl, idesc_bf16(NOUT * (n - 1)), 1u);
+                mma_bf16_on(on, dm, ga, b0 + (uint64_t)(2 * NOUT), idesc_bf16(NOUT), 0u);
+            } else {
+                mma_bf16_on(on, d, ga, bl, idn, 1u);
+            }
+#pragma unroll
+            for (int k = 1; k < 9 * L::kHalves; ++k) {
+                const int r = k / L::kHalves, h = k % L::kHalves;  // (dy, dx) and the half
+                const uint32_t ao = ((r / 3) * L::kRunB + (r % 3) * 16 + 2 * h * kPlaneB) >> 4;
+                mma_bf16_on(on, d, ga + ao, bl + ((k * L::kWBlk) >> 4), idn, 1u);
+                if (k == 3 * L::kHalves) commit();
+            }
+            csl = sl;
+            cacc = m - 2;
+            if (++m == nz + 2) {
+                m = 0;
+                u += gridDim.x;
+                if (u < U) {
+                    const Unit w = unit_of(a.N, a.tiles_x, a.unit_z, u);
+                    nz = w.z1 - w.z0;
+                }
+            }
+            if (++sl == kRing) {
+                sl = 0;
+                gph ^= 1u;
+            }
+        }
+        commit();
+        if (on) mma_commit(done);
+        __syncwarp();
+        mbar_wait(done, 0, a.err, 25);
+    } else if (warp < 4) {
         if (lane == 0) {
-            mbar_arrive_expect(wbar, (uint32_t)L::kWB);
-            for (int off = 0; off < L::kWB; off += 16384) {
-                const int nb = L::kWB - off < 16384 ? L::kWB - off : 16384;
-                bulk_load(wsm + off, a.w + off, (uint32_t)nb, wbar);
+            const int dy = warp - 1;
+            if (dy == 0) {
+                mbar_arrive_expect(wbar, (uint32_t)L::kWB);
+                for (int off = 0; off < L::kWB; off += 16384) {
+                    const int nb = L::kWB - off < 16384 ? L::kWB - off : 16384;
+                    bulk_load(wsm + off, a.w + off, (uint32_t)nb, wbar);
+                }
             }
             bool ok = true;
             int g = 0;
             for (long long u = blockIdx.x; ok && u < U; u += gridDim.x) {
-                int x0, y0, y1, z;
-                unit_of(a, u, x0, y0, y1, z);
-                for (int yy = y0 - 1; yy <= y1; ++yy, ++g) {
+                const Unit w = unit_of(a.N, a.tiles_x, a.unit_z, u);
+                for (int zz = w.z0 - 1; zz <= w.z1; ++zz, ++g) {
                     const int sl = g % kRing;
                     if (g >= kRing && !mbar_wait1(&empty[sl], ((g / kRing) - 1) & 1, a.err, 21)) {
                         ok = false;
                         break;
                     }
-                    uint8_t* gb = smem + sl * L::kGroupB;
-                    mbar_arrive_expect(&full[sl], (uint32_t)(3 * CIN8 * kRunPlaneB));
-                    for (int dz = 0; dz < 3; ++dz)
-                        tma_load_5d(gb + dz * L::kRunB, &a.in, 0, x0 - 1, yy, z + dz - 1, 0, &full[sl]);
-                }
-            }
-        }
-    } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = idesc_bf16(NOUT);
-            bool ok = mbar_wait1(wbar, 0, a.err, 22);
-            const uint64_t b0 = sdesc(smem_u32(wsm), NOUT * 16, 128);
-            const uint32_t rbase = smem_u32(smem);
-            int g = 0, k = 0;
-            for (long long u = blockIdx.x; ok && u < U; u += gridDim.x) {
-                int x0, y0, y1, z;
-                unit_of(a, u, x0, y0, y1, z);
-                const int ny = y1 - y0;
-                for (int i = 0; i < ny; ++i, ++k) {
-                    const int ac = k & 1;
-                    for (int j = 0; j < 3 && ok; ++j) {
-                        const int gg = g + i + j;
-                        ok = mbar_wait1(&full[gg % kRing], (gg / kRing) & 1, a.err, 23);
-                    }
-                    if (ok && k >= 2) ok = mbar_wait1(&acce[ac], ((k >> 1) - 1) & 1, a.err, 24);
-                    if (!ok) break;
-                    tc_fence_after();
-                    const uint32_t d = tmem + (uint32_t)(ac * 32);
-                    uint64_t ga[3];  // descriptors of the three row groups (start addresses differ)
+                    uint8_t* rb = smem + sl * L::kGroupB + dy * L::kRunB;
+                    mbar_arrive_expect(&full[sl], (uint32_t)(CIN8 * (kTileM + 2) * 16));
+                    // elements of the maps are half voxels (8 bytes); the run starts at x0 - 1
 #pragma unroll
-                    for (int j = 0; j < 3; ++j)
-                        ga[j] = sdesc(rbase + (uint32_t)(((g + i + j) % kRing) * L::kGroupB), kRunPlaneB, 128);
-#pragma unroll
-                    for (int tap = 0; tap < 27; ++tap) {
-#pragma unroll
-                        for (int h = 0; h < L::kHalves; ++h) {
-                            const uint32_t ao = ((tap / 9) * L::kRunB + (tap % 3) * 16 + 2 * h * kRunPlaneB) >> 4;
-                            const uint32_t bo = ((tap * L::kHalves + h) * L::kWBlk) >> 4;
-                            mma_bf16(d, ga[(tap / 3) % 3] + ao, b0 + bo, idesc, (tap | h) != 0 ? 1u : 0u);
-                        }
-                    }
-                    mma_commit(&accf[ac]);
-                    if (i < ny - 1) {
-                        mma_commit(&empty[(g + i) % kRing]);
-                    } else {
-                        for (int j = 0; j < 3; ++j) mma_commit(&empty[(g + i + j) % kRing]);
+                    for (int pl = 0; pl < CIN8; ++pl) {
+                        tma_load_4d(rb + pl * kPlaneB, &a.in.run, 2 * (w.x0 - 1), w.y + dy - 1, zz, pl, &full[sl]);
+                        tma_load_4d(rb + pl * kPlaneB + kTileM * 16, &a.in.tail, 2 * (w.x0 + kTileM - 1), w.y + dy - 1, zz, pl, &full[sl]);
                     }
                 }
-                g += ny + 2;
             }
-            mma_commit(done);
-            mbar_wait1(done, 0, a.err, 25);
         }
     } else {
-        const int q = warp & 3;
+        const int q = warp & 3, grp = (warp - 4) >> 2;  // TMEM lanes 32q.. are this warp's
         float bias[NOUT];
 #pragma unroll
         for (int n = 0; n < NOUT; ++n) bias[n] = a.bias[n];
-        int k = 0;
+        uint32_t phase = 0;
         bool ok = true;
         for (long long u = blockIdx.x; ok && u < U; u += gridDim.x) {
-            int x0, y0, y1, z;
-            unit_of(a, u, x0, y0, y1, z);
-            for (int y = y0; y < y1; ++y, ++k) {
-                const int ac = k & 1;
-                if (!mbar_wait(&accf[ac], (k >> 1) & 1, a.err, 26)) {
+            const Unit w = unit_of(a.N, a.tiles_x, a.unit_z, u);
+            const int x = w.x0 + 32 * q + lane;
+            for (int i = grp; i < w.z1 - w.z0; i += 2) {
+                TileIn<NOUT, MODE> in;
+                in.request(a, x, w.y, w.z0 + i);  // residual and mask planes on their way during the wait
+                if (!mbar_wait(&accf[i], (phase >> i) & 1u, a.err, 26)) {
                     ok = false;
                     break;
                 }
+                phase ^= 1u << i;
                 tc_fence_after();
                 uint32_t v[NOUT];
-                const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(ac * 32);
-                if constexpr (NOUT == 32) tmem_ld32(ta, v);
-                else tmem_ld16(ta, v);
+                const uint32_t ta = tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(i * NOUT);
+                tmem_ld32(ta, v);
                 tmem_wait_ld();
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&acce[ac]);
-                store_tile<NOUT, MODE>(a, v, bias, x0 + 32 * q + lane, y, z);
+                if (lane == 0) mbar_arrive(&acce[i]);
+                store_tile<NOUT, MODE>(a, v, bias, in, x, w.y, w.z0 + i);
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 1) {
+    if (warp == 0) {
         __syncwarp();
         tc_fence_after();
-        tmem_dealloc(tmem, 64);
+        tmem_dealloc(tmem, 512);
     }
 }
 
 // ---------------------------------------------------------------- weight gradients
-// k_wgrad (32 -> 32 layers, tcgen05): dW[co][ci][tap] = sum over voxels v of X[ci, v + tap] * G[co, v]
-// (X = the layer's input, G = the gradient of its output, zero outside the grid).  The voxels are
-// the K dimension, so both operands are read MN-major from the 8-channel planes as staged (8
-// channels of one voxel = 16 contiguous bytes, consecutive voxels 16 bytes apart: the canonical
-// no-swizzle MN-major layout, channel groups SBO apart, voxel groups of 8 LBO = 128 bytes apart).
-// Per tile (128 voxels of one x-line): the 9 runs of X (130 voxels, 4 planes) and the 128-voxel
-// run of G (4 planes); A = four consecutive runs r0..r0+3 as M = 128 rows (run, ci) (the runs of a
-// stage are 4 * 2080 bytes apart, so rows keep one stride), moved by dx voxels for tap dx; B = G.
-// 3 row groups x 3 dx x 8 blocks of 16 voxels = 72 MMAs per tile into 9 TMEM accumulators (288
-// columns) that persist over all tiles of the CTA; rows 9-11 of the last group read past the stage
-// into other staged data and are discarded.  At the end each CTA writes its partial sums.
-constexpr int kWgRunB = 4 * kRunPlaneB;            // 8320
-constexpr int kWgXB = 9 * kWgRunB;                  // 74,880
-constexpr int kWgGB = 4 * kTileM * 16;              // 8,192
-constexpr int kWgStageB = kWgXB + kWgGB;            // 83,072
-constexpr int kWgTail = 3 * kWgRunB;                // room for the discarded rows of the last stage
-constexpr int kWgBars = 2 * kWgStageB + kWgTail;
-constexpr int kWgBytes = kWgBars + 5 * 8 + 16;
+// k_wgrad (32 -> 32 layers, tcgen05): dW[co][ci][tap] = sum over voxels v of X[ci, v] * G[co, v - tap]
+// (X = the layer's input, G = the gradient of its output, zero outside the grid).  The voxels are the K
+// dimension, so both operands are read MN-major from the 8-channel planes as staged (8 channels of one
+// voxel = 16 contiguous bytes, consecutive voxels 16 bytes apart: the canonical no-swizzle MN-major
+// layout, channel groups SBO apart, voxel groups of 8 LBO = 128 bytes apart).  Per tile (128 voxels of one
+// x-line): A = a row group of X (the runs y-1, y, y+1 at one z) as M = 128 rows (dy, ci) (the rows past 96 are
+// whatever lies behind the group and are discarded), one of the three groups dz; B = three copies of the
+// G run moved by -1, 0, 1 voxels as N = 96 columns (dx, co).  3 dz x 8 blocks of 16 voxels = 24 MMAs
+// per tile into 3 TMEM accumulators that persist over all tiles of the CTA.  (As 72 MMAs of N = 32 with
+// A moved by dx voxels, off the 128-byte core matrices, and all 9 runs of X loaded per tile, a launch at
+// 96^3 took 206 us, 115 now.)  X's row groups go through the ring of the convolutions: units of up to
+// kUnitZ lines, each group loaded once per unit.  At the end each CTA writes its partial sums.
+constexpr int kWgRing = 6;
+constexpr int kWgGroupB = 3 * 4 * kRunPlaneB;       // one row group of X
+constexpr int kWgGB = 3 * 4 * kRunPlaneB;           // the three copies of the G run
+constexpr int kWgBars = kWgRing * kWgGroupB + 2 * kWgGB;
+constexpr int kWgBytes = kWgBars + (2 * kWgRing + 5) * 8 + 16;
 
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int n) {
     return idesc_bf16(n) | (1u << 15) | (1u << 16);
 }
 
 struct WgradArgs {
-    CUtensorMap x;  // {8, N, N, N, 4}, box {8, 130, 1, 1, 4}
-    CUtensorMap g;  // {8, N, N, N, 4}, box {8, 128, 1, 1, 4}
-    float* partial; // [gridDim.x][32 co][32 ci][27]
-    int N, tiles_x;
-    long long tiles;
+    CUtensorMap x, g;  // plane_map of X and of G (4 planes each)
+    float* partial;    // [gridDim.x][32 co][32 ci][27]
+    int N, tiles_x, unit_z;
     int* err;
 };
 
 __global__ void __launch_bounds__(192, 1) k_wgrad(const __grid_constant__ WgradArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
+    uint8_t* gsm = smem + kWgRing * kWgGroupB;
     uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kWgBars);
-    uint64_t* full = bars;
-    uint64_t* empty = bars + 2;
-    uint64_t* done = bars + 4;
-    uint32_t* tslot = reinterpret_cast<uint32_t*>(bars + 5);
+    uint64_t* full = bars;              // [kWgRing] row group of X loaded
+    uint64_t* empty = bars + kWgRing;     // [kWgRing]
+    uint64_t* gfull = bars + 2 * kWgRing; // [2] copies of G loaded
+    uint64_t* gempty = gfull + 2;       // [2]
+    uint64_t* done = gempty + 2;
+    uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 2; ++i) {
+        for (int i = 0; i < kWgRing; ++i) {
             mbar_init(&full[i], 1);
             mbar_init(&empty[i], 1);
+        }
+        for (int i = 0; i < 2; ++i) {
+            mbar_init(&gfull[i], 1);
+            mbar_init(&gempty[i], 1);
         }
         mbar_init(done, 1);
         fence_mbar_init();
@@ -570,70 +521,105 @@ __global__ void __launch_bounds__(192, 1) k_wgrad(const __grid_constant__ WgradA
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
-    const long long T = a.tiles;
-    ConvArgs geo{};
-    geo.N = a.N;
-    geo.tiles_x = a.tiles_x;
+    const long long U = unit_count(a.N, a.tiles_x, a.unit_z);
     if (warp == 0) {
         if (lane == 0) {
-            int k = 0;
-            for (long long t = blockIdx.x; t < T; t += gridDim.x, ++k) {
-                const int s = k & 1;
-                if (k >= 2 && !mbar_wait1(&empty[s], ((k >> 1) - 1) & 1, a.err, 31)) break;
-                int x0, y, z;
-                tile_of(geo, t, x0, y, z);
-                uint8_t* st = smem + s * kWgStageB;
-                mbar_arrive_expect(&full[s], (uint32_t)(kWgXB + kWgGB));
-                for (int r = 0; r < 9; ++r)
-                    tma_load_5d(st + r * kWgRunB, &a.x, 0, x0 - 1, y + r % 3 - 1, z + r / 3 - 1, 0, &full[s]);
-                tma_load_5d(st + kWgXB, &a.g, 0, x0, y, z, 0, &full[s]);
+            bool ok = true;
+            int g = 0, k = 0;
+            for (long long u = blockIdx.x; ok && u < U; u += gridDim.x) {
+                const Unit w = unit_of(a.N, a.tiles_x, a.unit_z, u);
+                    for (int zz = w.z0 - 1; ok && zz <= w.z1; ++zz, ++g) {
+                        const int sl = g % kWgRing;
+                        if (g >= kWgRing && !mbar_wait1(&empty[sl], ((g / kWgRing) - 1) & 1, a.err, 31)) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_arrive_expect(&full[sl], (uint32_t)kWgGroupB);
+                        for (int dy = 0; dy < 3; ++dy)
+                            tma_load_4d(smem + sl * kWgGroupB + dy * 4 * kRunPlaneB, &a.x, 2 * w.x0, w.y + dy - 1, zz, 0, &full[sl]);
+                        if (zz < w.z0 || zz >= w.z1) continue;
+                        const int s = k & 1;
+                        if (k >= 2 && !mbar_wait1(&gempty[s], ((k >> 1) - 1) & 1, a.err, 34)) {
+                            ok = false;
+                            break;
+                        }
+                        mbar_arrive_expect(&gfull[s], (uint32_t)kWgGB);
+                        // copy dx holds G[v + 1 - dx]
+                        for (int dx = 0; dx < 3; ++dx)
+                            tma_load_4d(gsm + s * kWgGB + dx * 4 * kRunPlaneB, &a.g, 2 * (w.x0 + 1 - dx), w.y, zz, 0, &gfull[s]);
+                        ++k;
+                    }
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
-            constexpr uint32_t idesc = idesc_bf16_mn(32);
-            int k = 0;
-            for (long long t = blockIdx.x; t < T; t += gridDim.x, ++k) {
-                const int s = k & 1;
-                if (!mbar_wait1(&full[s], (k >> 1) & 1, a.err, 32)) break;
-                tc_fence_after();
-                const uint32_t sb = smem_u32(smem + s * kWgStageB);
-                const uint64_t a0 = sdesc(sb, 128, kRunPlaneB);         // LBO = voxel groups, SBO = channel groups
-                const uint64_t b0 = sdesc(sb + kWgXB, 128, kTileM * 16);
-#pragma unroll
-                for (int rg = 0; rg < 3; ++rg)
-#pragma unroll
-                    for (int dx = 0; dx < 3; ++dx)
-#pragma unroll
-                        for (int kb = 0; kb < 8; ++kb) {
-                            const uint32_t ao = (4 * rg * kWgRunB + (dx + 16 * kb) * 16) >> 4;
-                            const uint32_t bo = (16 * kb * 16) >> 4;
-                            mma_bf16(tmem + (uint32_t)(32 * (3 * rg + dx)), a0 + ao, b0 + bo, idesc,
-                                     (k > 0 || kb > 0) ? 1u : 0u);
-                        }
-                mma_commit(&empty[s]);
+        // the whole warp runs the loop, one lane issues; hand-overs are committed a few MMAs into the next
+        // line (see k_conv3)
+        constexpr uint32_t idesc = idesc_bf16_mn(96);
+        const uint32_t on = elect_one();
+        bool ok = true;
+        int g = 0, k = 0;
+        int crel = 0, cg = 0, cs = -1;  // the line before: groups to release from group cg on, its copies of G
+        auto commit = [&] {
+            if (on && cs >= 0) {
+                mma_commit(&gempty[cs]);
+                for (int j = 0; j < crel; ++j) mma_commit(&empty[(cg + j) % kWgRing]);
             }
-            mma_commit(done);
+            __syncwarp();
+        };
+        for (long long u = blockIdx.x; ok && u < U; u += gridDim.x) {
+            const Unit w = unit_of(a.N, a.tiles_x, a.unit_z, u);
+            const int nz = w.z1 - w.z0;
+            for (int i = 0; i < nz; ++i, ++k) {
+                const int s = k & 1;
+                if (i == 0) {
+                    // the first two groups of a unit may wait for slots that the last line still holds
+                    commit();
+                    cs = -1;
+                }
+                for (int j = i == 0 ? 0 : 2; j < 3 && ok; ++j) {
+                    const int gg = g + i + j;
+                    ok = mbar_wait(&full[gg % kWgRing], (gg / kWgRing) & 1, a.err, 32);
+                }
+                if (ok) ok = mbar_wait(&gfull[s], (k >> 1) & 1, a.err, 35);
+                if (!ok) break;
+                tc_fence_after();
+                const uint64_t b0 = sdesc(smem_u32(gsm + s * kWgGB), 128, kRunPlaneB);
+                const uint32_t acc = k > 0 ? 1u : 0u;
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    const uint64_t a0 = sdesc(smem_u32(smem) + (uint32_t)(((g + i + j) % kWgRing) * kWgGroupB), 128, kRunPlaneB);
+#pragma unroll
+                    for (int kb = 0; kb < 8; ++kb) {
+                        mma_bf16_on(on, tmem + (uint32_t)(128 * j), a0 + 16 * kb, b0 + 16 * kb, idesc, kb > 0 ? 1u : acc);
+                        if (j == 0 && kb == 3) commit();
+                    }
+                }
+                cs = s;
+                cg = g + i;
+                crel = i < nz - 1 ? 1 : 3;
+            }
+            g += nz + 2;
         }
+        commit();
+        if (on) mma_commit(done);
+        __syncwarp();
+        mbar_wait(done, 0, a.err, 36);
     } else {
-        // read the 9 accumulators once every MMA of the CTA has finished
+        // read the 3 accumulators once every MMA of the CTA has finished
         const int q = warp & 3;
-        if (mbar_wait(done, 0, a.err, 33, 1 << 26)) {
+        if (mbar_wait(done, 0, a.err, 33, 1 << 26) && q < 3) {
             tc_fence_after();
             float* out = a.partial + (size_t)blockIdx.x * (32 * 32 * 27);
-            const bool any = blockIdx.x < T;
+            const bool anz = blockIdx.x < U;
             for (int j = 0; j < 9; ++j) {
-                const int rg = j / 3, dx = j % 3;
+                const int dz = j / 3, dx = j % 3;
                 uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(32 * j), v);
+                tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(128 * dz + 32 * dx), v);
                 tmem_wait_ld();
-                const int r = 4 * rg + q;  // lane 32q + ci is row (run r, ci)
-                if (r < 9) {
-                    const int tap = 3 * r + dx;
+                const int tap = 9 * dz + 3 * q + dx;  // lane 32q + ci is row (dy = q, ci)
 #pragma unroll
-                    for (int co = 0; co < 32; ++co)
-                        out[((size_t)co * 32 + lane) * 27 + tap] = any ? __uint_as_float(v[co]) : 0.f;
-                }
+                for (int co = 0; co < 32; ++co)
+                    out[((size_t)co * 32 + lane) * 27 + tap] = anz ? __uint_as_float(v[co]) : 0.f;
             }
         }
     }
@@ -827,8 +813,9 @@ __global__ void k_pack_w(const float* W, int cin, int cout, int cin8, int nout, 
     const int halves = cin8 / 2;
     const int n_img = 27 * halves * 2 * nout * 8;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_img; i += gridDim.x * blockDim.x) {
-        const int e = i % 8, n = (i / 8) % nout, kc = (i / (8 * nout)) % 2, h = (i / (16 * nout)) % halves;
-        const int tap = i / (16 * nout * halves);
+        const int e = i % 8, n = (i / 8) % nout, dz = 2 - (i / (8 * nout)) % 3, kc = (i / (24 * nout)) % 2;
+        const int h = (i / (48 * nout)) % halves, r = i / (48 * nout * halves);  // r = 3 dy + dx
+        const int tap = 9 * dz + r;
         const int k = 16 * h + 8 * kc + e;  // input channel of the packed convolution
         float v = 0.f;
         if (!transpose) {
@@ -914,7 +901,7 @@ struct LayerShape {
 constexpr LayerShape kShape[kLayers] = {
     {kInCh, kHidden, 2, 32},   {kHidden, kHidden, 4, 32}, {kHidden, kHidden, 4, 32}, {kHidden, kHidden, 4, 32},
     {kHidden, kHidden, 4, 32}, {kHidden, kHidden, 4, 32}, {kHidden, kHidden, 4, 32}, {kHidden, kHidden, 4, 32},
-    {kHidden, kHidden, 4, 32}, {kHidden, 1, 4, 16}};
+    {kHidden, kHidden, 4, 32}, {kHidden, 1, 4, 32}};
 
 }  // namespace
 
@@ -937,7 +924,7 @@ struct TrainState {
     uint4* tb[4] = {};
     uint4 *gh = nullptr, *gu = nullptr, *gd = nullptr;
     float* tgt = nullptr;        // the plain solver's field after the substeps (pitched)
-    CUtensorMap mh[5], mt[4], mgd, mgh, mgu, mgh_g, mgu_g;
+    PlaneMaps mh[5], mt[4], mgd, mgh, mgu;
     int step = 0;
 };
 
@@ -957,7 +944,7 @@ struct SurrogateState {
     float* backup = nullptr;    // field before the step (pitched)
     unsigned* dmax = nullptr;   // judge scratch
     unsigned* hmax = nullptr;   // pinned host copy
-    CUtensorMap map_in, map_h, map_t;
+    PlaneMaps map_in, map_h, map_t;
     struct TrainState* train = nullptr;
 };
 
@@ -987,7 +974,7 @@ void surrogate_free(gell_ctx* c) {
     }
 }
 
-static gell_status plane_map(gell_ctx* c, CUtensorMap* m, void* base, int planes, int box_x = kRunVox) {
+static gell_status plane_map(gell_ctx* c, PlaneMaps* m, void* base, int planes) {
     static PFN_cuTensorMapEncodeTiled_v12000 encode = nullptr;
     if (!encode) {
         cudaDriverEntryPointQueryResult q;
@@ -998,19 +985,23 @@ static gell_status plane_map(gell_ctx* c, CUtensorMap* m, void* base, int planes
         encode = (PFN_cuTensorMapEncodeTiled_v12000)fn;
     }
     const cuuint64_t N = (cuuint64_t)c->g.N;
-    const cuuint64_t dims[5] = {8, N, N, N, (cuuint64_t)planes};
-    const cuuint64_t strides[4] = {16, 16 * N, 16 * N * N, 16 * N * N * N};
-    const cuuint32_t box[5] = {8, (cuuint32_t)box_x, 1, 1, (cuuint32_t)planes};
-    const cuuint32_t es[5] = {1, 1, 1, 1, 1};
-    CUresult r = encode(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 5, base, dims, strides, box, es,
-                        CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                        CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    // half voxels (8 bytes) as elements: a run of 128 voxels is one row of a box, 256 elements
+    const cuuint64_t dims[4] = {2 * N, N, N, (cuuint64_t)planes};
+    const cuuint64_t strides[3] = {16 * N, 16 * N * N, 16 * N * N * N};
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    CUresult r = CUDA_SUCCESS;
+    for (int k = 0; k < 3 && r == CUDA_SUCCESS; ++k) {
+        const cuuint32_t box[4] = {k == 1 ? 4u : 2u * kTileM, 1, 1, k == 2 ? (cuuint32_t)planes : 1u};
+        r = encode(k == 0 ? &m->run : k == 1 ? &m->tail : &m->all, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, base, dims, strides, box, es,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    }
     if (r != CUDA_SUCCESS) return fail(c, GELL_ERR_CUDA, "cuTensorMapEncodeTiled (planes) failed (" + std::to_string((int)r) + ")");
     return GELL_OK;
 }
 
 // Pack one layer's fp32 weights W[cout][cin][3][3][3] (PyTorch conv3d order, kz kz ky kx = dz dy dx
-// + 1) into the shared-memory image: block (tap, half) holds [kc][n][8] with input channel
+// + 1) into the shared-memory image: block (dy, dx, half) holds [kc][2 - dz][n][8] with input channel
 // 16*half + 8*kc + e and output channel n; padding channels are zero.
 static void pack_layer(const float* W, const LayerShape& s, std::vector<uint16_t>& img) {
     const int halves = s.cin8 / 2;
@@ -1030,23 +1021,32 @@ static void pack_layer(const float* W, const LayerShape& s, std::vector<uint16_t
                         const int ci = 16 * h + 8 * kc + e;
                         float v = 0.f;
                         if (n < s.cout && ci < s.cin) v = W[((size_t)n * s.cin + ci) * 27 + tap];
-                        img[((((size_t)tap * halves + h) * 2 + kc) * s.nout + n) * 8 + e] = bf(v);
+                        img[(((((size_t)(tap % 9) * halves + h) * 2 + kc) * 3 + 2 - tap / 9) * s.nout + n) * 8 + e] = bf(v);
                     }
 }
 
+// Lines per unit: as many as possible (a unit loads two row groups more than it has lines), but few enough
+// that the units fill the last round of CTAs; the cost of a round is its lines plus those two groups.
+static int unit_lines(int N, int sms) {
+    int best = kUnitZ;
+    long long cost = -1;
+    for (int y = kUnitZ; y >= 4; --y) {
+        const long long units = (long long)((N + kTileM - 1) / kTileM) * ((N + y - 1) / y) * N, rounds = (units + sms - 1) / sms;
+        if (cost < 0 || rounds * (y + 2) < cost) {
+            cost = rounds * (y + 2);
+            best = y;
+        }
+    }
+    return best;
+}
+
 template <int CIN8, int NOUT, int MODE>
-static gell_status launch_conv(gell_ctx* c, const char* name, const CUtensorMap& in, const uint8_t* w, const float* bias,
+static gell_status launch_conv(gell_ctx* c, const char* name, const PlaneMaps& in, const uint8_t* w, const float* bias,
                                uint4* out, const uint4* res, const uint4* aux, float* fout, const float* fin, float scale,
                                float bval) {
     using L = ConvSmem<CIN8, NOUT>;
-    using R = RingSmem<CIN8, NOUT>;
     // the shared-memory opt-in is a per-device attribute; setting it is cheap, so every launch does
-    if (c->conv_ring)
-        GELL_CUDA(c, cudaFuncSetAttribute(k_conv3_ring<CIN8, NOUT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          R::kBytes));
-    else
-        GELL_CUDA(c, cudaFuncSetAttribute(k_conv3<CIN8, NOUT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          L::kBytes));
+    GELL_CUDA(c, cudaFuncSetAttribute(k_conv3<CIN8, NOUT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
     ConvArgs a{};
     a.in = in;
     a.w = w;
@@ -1061,20 +1061,15 @@ static gell_status launch_conv(gell_ctx* c, const char* name, const CUtensorMap&
     a.PN = c->g.PN;
     a.nvox = c->nvox;
     a.tiles_x = (c->g.N + kTileM - 1) / kTileM;
-    a.tiles = (long long)a.tiles_x * c->g.N * c->g.N;
     a.scale = scale;
     a.bval = bval;
     a.err = c->dev_err;
     int sms = 0;
     GELL_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-    if (c->conv_ring) {
-        const long long units = (long long)a.tiles_x * ((c->g.N + kUnitY - 1) / kUnitY) * c->g.N;
-        const int grid = (int)(units < sms ? units : sms);
-        GELL_KERNEL(c, name, (k_conv3_ring<CIN8, NOUT, MODE><<<grid, 192, R::kBytes, c->stream>>>(a)));
-    } else {
-        const int grid = (int)(a.tiles < sms ? a.tiles : sms);
-        GELL_KERNEL(c, name, (k_conv3<CIN8, NOUT, MODE><<<grid, 192, L::kBytes, c->stream>>>(a)));
-    }
+    a.unit_z = unit_lines(c->g.N, sms);
+    const long long units = (long long)a.tiles_x * ((c->g.N + a.unit_z - 1) / a.unit_z) * c->g.N;
+    const int grid = (int)(units < sms ? units : sms);
+    GELL_KERNEL(c, name, (k_conv3<CIN8, NOUT, MODE><<<grid, kConvThreads, L::kBytes, c->stream>>>(a)));
     return GELL_OK;
 }
 
@@ -1126,7 +1121,7 @@ static gell_status run_layers(gell_ctx* c, int sub, SurrogateState* S, int layer
         if (l == 0)
             st = launch_conv<2, 32, kRelu>(c, "k_conv3_in", S->map_in, w, bi, S->h, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f);
         else if (l == kLayers - 1)
-            st = launch_conv<4, 16, kField>(c, "k_conv3_out", S->map_h, w, bi, nullptr, nullptr, nullptr, S->ph, Su.p, scale, b);
+            st = launch_conv<4, 32, kField>(c, "k_conv3_out", S->map_h, w, bi, nullptr, nullptr, nullptr, S->ph, Su.p, scale, b);
         else if (l & 1)
             st = launch_conv<4, 32, kRelu>(c, "k_conv3_hidden", S->map_h, w, bi, S->t, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f);
         else
@@ -1139,7 +1134,7 @@ static gell_status infer(gell_ctx* c, int sub, SurrogateState* S) { return run_l
 // Shapes of the data-gradient convolution of layer l: input planes (the layer's outputs, padded to
 // 16 channels) and outputs (the layer's inputs).
 static int dgrad_cin8(int l) { return kShape[l].cout <= 16 ? 2 : 4; }
-static int dgrad_nout(int l) { return kShape[l].cin <= 16 ? 16 : 32; }
+static int dgrad_nout(int) { return 32; }
 
 static gell_status repack(gell_ctx* c, SurrogateState* S) {
     TrainState* T = S->train;
@@ -1160,24 +1155,25 @@ static int thin_blocks() { return 148 * 4; }
 
 // Weight gradient of layer l into T->grad (the layer's block): tcgen05 for the 32 -> 32 layers,
 // CUDA cores for the thin first and last layers; bias gradient = per-channel sums of G.
-static gell_status wgrad_layer(gell_ctx* c, SurrogateState* S, int l, const CUtensorMap* xmap, const uint4* X,
-                               const CUtensorMap* gmap, const uint4* G, int gplanes) {
+static gell_status wgrad_layer(gell_ctx* c, SurrogateState* S, int l, const PlaneMaps* xmap, const uint4* X,
+                               const PlaneMaps* gmap, const uint4* G, int gplanes) {
     TrainState* T = S->train;
     const LayerShape& sh = kShape[l];
     const int N = c->g.N;
     const int nw = sh.cout * sh.cin * 27;
     if (sh.cin == kHidden && sh.cout == kHidden) {
         WgradArgs a{};
-        a.x = *xmap;
-        a.g = *gmap;
+        a.x = xmap->all;
+        a.g = gmap->all;
         a.partial = T->partial;
         a.N = N;
         a.tiles_x = (N + kTileM - 1) / kTileM;
-        a.tiles = (long long)a.tiles_x * N * N;
         a.err = c->dev_err;
         int sms = 0;
         GELL_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-        const int grid = (int)(a.tiles < sms ? a.tiles : sms);
+        a.unit_z = unit_lines(N, sms);
+        const long long units = (long long)a.tiles_x * ((N + a.unit_z - 1) / a.unit_z) * N;
+        const int grid = (int)(units < sms ? units : sms);
         GELL_CUDA(c, cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgBytes));
         GELL_KERNEL(c, "k_wgrad", (k_wgrad<<<grid, 192, kWgBytes, c->stream>>>(a)));
         GELL_KERNEL(c, "k_sum_partials", (k_sum_partials<<<(nw + 255) / 256, 256, 0, c->stream>>>(T->partial, grid, nw, nw,
@@ -1235,7 +1231,7 @@ static gell_status train_pair(gell_ctx* c, int sub, SurrogateState* S, float lr,
                                                T->hb[k + 1], T->hb[k], nullptr, nullptr, nullptr, 0.f, 0.f);
     }
     if (st == GELL_OK)
-        st = launch_conv<4, 16, kField>(c, "k_conv3_out", T->mh[4], S->w[9], S->bias[9], nullptr, nullptr, nullptr, S->ph,
+        st = launch_conv<4, 32, kField>(c, "k_conv3_out", T->mh[4], S->w[9], S->bias[9], nullptr, nullptr, nullptr, S->ph,
                                         Su.p, scale, b);
     if (st != GELL_OK) return st;
 
@@ -1251,11 +1247,11 @@ static gell_status train_pair(gell_ctx* c, int sub, SurrogateState* S, float lr,
     st = launch_conv<2, 32, kLinear>(c, "k_conv3_dgrad", T->mgd, T->wt[9], T->zero_bias, T->gh, nullptr, nullptr, nullptr,
                                      nullptr, 0.f, 0.f);
     for (int k = 3; k >= 0 && st == GELL_OK; --k) {
-        if ((st = wgrad_layer(c, S, 2 * k + 2, &T->mt[k], T->tb[k], &T->mgh_g, T->gh, 4)) != GELL_OK) return st;
+        if ((st = wgrad_layer(c, S, 2 * k + 2, &T->mt[k], T->tb[k], &T->mgh, T->gh, 4)) != GELL_OK) return st;
         st = launch_conv<4, 32, kMask>(c, "k_conv3_dgrad", T->mgh, T->wt[2 * k + 2], T->zero_bias, T->gu, nullptr,
                                        T->tb[k], nullptr, nullptr, 0.f, 0.f);
         if (st != GELL_OK) return st;
-        if ((st = wgrad_layer(c, S, 2 * k + 1, &T->mh[k], T->hb[k], &T->mgu_g, T->gu, 4)) != GELL_OK) return st;
+        if ((st = wgrad_layer(c, S, 2 * k + 1, &T->mh[k], T->hb[k], &T->mgu, T->gu, 4)) != GELL_OK) return st;
         if (k > 0)
             st = launch_conv<4, 32, kResidual>(c, "k_conv3_dgrad", T->mgu, T->wt[2 * k + 1], T->zero_bias, T->gh, T->gh,
                                                nullptr, nullptr, nullptr, 0.f, 0.f);
@@ -1432,8 +1428,6 @@ gell_status gell_surrogate_train_init(gell_ctx* c, int sub, const float* weights
         if (st == GELL_OK) st = plane_map(c, &T->mgd, T->gd, 2);
         if (st == GELL_OK) st = plane_map(c, &T->mgh, T->gh, 4);
         if (st == GELL_OK) st = plane_map(c, &T->mgu, T->gu, 4);
-        if (st == GELL_OK) st = plane_map(c, &T->mgh_g, T->gh, 4, kTileM);
-        if (st == GELL_OK) st = plane_map(c, &T->mgu_g, T->gu, 4, kTileM);
         if (st != GELL_OK) return st;
     }
     TrainState* T = S->train;

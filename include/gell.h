@@ -308,9 +308,8 @@ enum {
  * their own (forked from and joined back to the context's stream), so that one substrate's sweep
  * fills the SMs another's leaves idle at its start and end (the plane sweeps take every substrate in
  * one launch instead).  Results are identical. */
-/* GELL_OPT_CONV_RING (0 or 1, default 1): the surrogate's convolutions keep the input rows of
- * consecutive lines in a ring of shared-memory slots (each row read from L2 once per unit of 32
- * lines) instead of loading all nine rows per tile; the results are the same. */
+/* GELL_OPT_CONV_RING: accepted and without effect (the surrogate's convolutions have one form, which
+ * passes the input lines through a ring of shared-memory slots). */
 /* GELL_OPT_SWEEP_WARPS (0..4, default 0): line tiles (compute warps) per CTA of the line-tile sweeps;
  * 0 = as many as shared memory holds.  Fewer give more, smaller CTAs, which can fill the GPU
  * better for small grids run side by side (the ensemble tuner tries them).  Results do not change. */
