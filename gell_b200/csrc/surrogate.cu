@@ -94,15 +94,7 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t addr, uint32_t lbo, uint32_t 
 __host__ __device__ constexpr uint32_t idesc_bf16(int n) {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
-__device__ __forceinline__ void mma_bf16(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d),
-        "l"(a), "l"(b), "r"(idesc), "r"(acc)
-        : "memory");
-}
-// The same, issued by the lanes with `on` set of a warp that runs the whole loop together: operands that
+// One MMA, issued by the lanes with `on` set of a warp that runs the whole loop together: operands that
 // are uniform over the warp then stay in uniform registers, where the instruction wants them.  (From
 // inside a one-lane branch each operand is moved there again: 75 cycles an MMA.)
 __device__ __forceinline__ void mma_bf16_on(uint32_t on, uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
@@ -135,6 +127,14 @@ __device__ __forceinline__ void tmem_ld32(uint32_t a, uint32_t (&v)[32]) {
           "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
           "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
           "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+        : "r"(a));
+}
+
+__device__ __forceinline__ void tmem_ld16(uint32_t a, uint32_t (&v)[16]) {  // 16 columns
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
         : "r"(a));
 }
 
@@ -464,44 +464,67 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv3(const __grid_constant
 }
 
 // ---------------------------------------------------------------- weight gradients
-// k_wgrad (32 -> 32 layers, tcgen05): dW[co][ci][tap] = sum over voxels v of X[ci, v] * G[co, v - tap]
-// (X = the layer's input, G = the gradient of its output, zero outside the grid).  The voxels are the K
-// dimension, so both operands are read MN-major from the 8-channel planes as staged (8 channels of one
-// voxel = 16 contiguous bytes, consecutive voxels 16 bytes apart: the canonical no-swizzle MN-major
-// layout, channel groups SBO apart, voxel groups of 8 LBO = 128 bytes apart).  Per tile (128 voxels of one
-// x-line): A = a row group of X (the runs y-1, y, y+1 at one z) as M = 128 rows (dy, ci) (the rows past 96 are
-// whatever lies behind the group and are discarded), one of the three groups dz; B = three copies of the
-// G run moved by -1, 0, 1 voxels as N = 96 columns (dx, co).  3 dz x 8 blocks of 16 voxels = 24 MMAs
-// per tile into 3 TMEM accumulators that persist over all tiles of the CTA.  (As 72 MMAs of N = 32 with
-// A moved by dx voxels, off the 128-byte core matrices, and all 9 runs of X loaded per tile, a launch at
-// 96^3 took 206 us, 115 now.)  X's row groups go through the ring of the convolutions: units of up to
-// kUnitZ lines, each group loaded once per unit.  At the end each CTA writes its partial sums.
+// k_wgrad (tcgen05): S[t][b][a] = sum over voxels v of A[a, v] * B[b, v - t], t the 27 taps, A of 4 planes
+// (32 channels), B of BP planes, zero outside the grid.  With A = the layer's input and B = the gradient of
+// its output this is dW[b][a][t]; the first layer, whose input has 3 channels, takes A = the gradient and
+// B = its input, which is dW[a][b][-t].  The voxels are the K dimension, so both operands are read MN-major
+// from the 8-channel planes as staged (8 channels of one voxel = 16 contiguous bytes, consecutive voxels 16
+// bytes apart: the canonical no-swizzle MN-major layout, channel groups SBO apart, voxel groups of 8 LBO =
+// 128 bytes apart).  Per tile (128 voxels of one x-line): a row group of A (the runs y-1, y, y+1 at one z)
+// as M = 128 rows (dy, a) (the rows past 96 are whatever lies behind the group and are discarded), one of
+// the three groups dz; three copies of the B run moved by -1, 0, 1 voxels as N = 24 BP columns (dx, b).
+// 3 dz x 8 blocks of 16 voxels = 24 MMAs per tile into 3 accumulators.  A's row groups go through a ring:
+// units of up to kUnitZ lines, each group loaded once per unit.  At the end each CTA writes its sums.
+//
+// The tensor cores drop what lies below the accumulator's last bit, so the error grows with the number of
+// MMAs in a chain: over all of a CTA's lines it came to 6e-5 of a 32 -> 32 layer's gradient at 128^3.  Three
+// reader warps per dz therefore take the accumulators over into fp32 sums in registers: for B of 2 planes
+// after every line (two sets in turn, 8 MMAs a chain: 2e-7 of the gradient, which sums on the CUDA cores had
+// to 4e-7), for B of 4 planes (288 columns, one set fits tensor memory, so that the MMAs wait) two thirds
+// through the CTA's units and at the end.
+//
+// (As 72 MMAs of N = 32 with A moved by dx voxels, off the 128-byte core matrices, all 9 runs of the input
+// loaded per tile and partial sums written 108 bytes apart, a 32 -> 32 launch at 96^3 took 206 us, 106 now;
+// the first and last layers took 670 us each on the CUDA cores, 106 now.)
+constexpr int kWgPart = 27 * 32 * 32;  // floats of one CTA's partial sums, at most
+constexpr int kWgCtas = 148;           // CTAs at most (room for their partial sums)
 constexpr int kWgRing = 6;
-constexpr int kWgGroupB = 3 * 4 * kRunPlaneB;       // one row group of X
-constexpr int kWgGB = 3 * 4 * kRunPlaneB;           // the three copies of the G run
-constexpr int kWgBars = kWgRing * kWgGroupB + 2 * kWgGB;
-constexpr int kWgBytes = kWgBars + (2 * kWgRing + 5) * 8 + 16;
+constexpr int kWgThreads = 448;        // loads, MMAs, 3 x 4 reader warps
+template <int BP>
+struct WgradSmem {
+    static constexpr int kGroupB = 12 * kRunPlaneB;  // one row group of A
+    static constexpr int kCopyB = 3 * BP * kRunPlaneB;  // the three copies of the B run
+    // the operand A spans 16 planes from a group's start: with the copies of B behind the ring, always inside
+    static constexpr int kBars = kWgRing * kGroupB + 2 * kCopyB;
+    static constexpr int kBytes = kBars + (2 * kWgRing + 9) * 8 + 16;
+    static constexpr int kCols = 24 * BP;        // columns of one dz
+    static constexpr int kSets = BP == 2 ? 2 : 1;  // sets of accumulators
+};
 
 __host__ __device__ constexpr uint32_t idesc_bf16_mn(int n) {
     return idesc_bf16(n) | (1u << 15) | (1u << 16);
 }
 
 struct WgradArgs {
-    CUtensorMap x, g;  // plane_map of X and of G (4 planes each)
-    float* partial;    // [gridDim.x][32 co][32 ci][27]
+    CUtensorMap a, b;  // plane_map of A and of B
+    float* partial;    // [gridDim.x][27][8 BP][32]
     int N, tiles_x, unit_z;
     int* err;
 };
 
-__global__ void __launch_bounds__(192, 1) k_wgrad(const __grid_constant__ WgradArgs a) {
+template <int BP>
+__global__ void __launch_bounds__(kWgThreads, 1) k_wgrad(const __grid_constant__ WgradArgs a) {
+    using L = WgradSmem<BP>;
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t* gsm = smem + kWgRing * kWgGroupB;
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + kWgBars);
-    uint64_t* full = bars;              // [kWgRing] row group of X loaded
+    uint8_t* bsm = smem + kWgRing * L::kGroupB;
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem + L::kBars);
+    uint64_t* full = bars;                // [kWgRing] row group of A loaded
     uint64_t* empty = bars + kWgRing;     // [kWgRing]
-    uint64_t* gfull = bars + 2 * kWgRing; // [2] copies of G loaded
-    uint64_t* gempty = gfull + 2;       // [2]
-    uint64_t* done = gempty + 2;
+    uint64_t* bfull = bars + 2 * kWgRing; // [2] copies of B loaded
+    uint64_t* bempty = bfull + 2;         // [2]
+    uint64_t* sfull = bempty + 2;         // [2] a set's chain is complete
+    uint64_t* sread = sfull + 2;          // [2] ... and has been read (9 warps)
+    uint64_t* done = sread + 2;
     uint32_t* tslot = reinterpret_cast<uint32_t*>(done + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
@@ -510,8 +533,10 @@ __global__ void __launch_bounds__(192, 1) k_wgrad(const __grid_constant__ WgradA
             mbar_init(&empty[i], 1);
         }
         for (int i = 0; i < 2; ++i) {
-            mbar_init(&gfull[i], 1);
-            mbar_init(&gempty[i], 1);
+            mbar_init(&bfull[i], 1);
+            mbar_init(&bempty[i], 1);
+            mbar_init(&sfull[i], 1);
+            mbar_init(&sread[i], 9);
         }
         mbar_init(done, 1);
         fence_mbar_init();
@@ -528,41 +553,44 @@ __global__ void __launch_bounds__(192, 1) k_wgrad(const __grid_constant__ WgradA
             int g = 0, k = 0;
             for (long long u = blockIdx.x; ok && u < U; u += gridDim.x) {
                 const Unit w = unit_of(a.N, a.tiles_x, a.unit_z, u);
-                    for (int zz = w.z0 - 1; ok && zz <= w.z1; ++zz, ++g) {
-                        const int sl = g % kWgRing;
-                        if (g >= kWgRing && !mbar_wait1(&empty[sl], ((g / kWgRing) - 1) & 1, a.err, 31)) {
-                            ok = false;
-                            break;
-                        }
-                        mbar_arrive_expect(&full[sl], (uint32_t)kWgGroupB);
-                        for (int dy = 0; dy < 3; ++dy)
-                            tma_load_4d(smem + sl * kWgGroupB + dy * 4 * kRunPlaneB, &a.x, 2 * w.x0, w.y + dy - 1, zz, 0, &full[sl]);
-                        if (zz < w.z0 || zz >= w.z1) continue;
-                        const int s = k & 1;
-                        if (k >= 2 && !mbar_wait1(&gempty[s], ((k >> 1) - 1) & 1, a.err, 34)) {
-                            ok = false;
-                            break;
-                        }
-                        mbar_arrive_expect(&gfull[s], (uint32_t)kWgGB);
-                        // copy dx holds G[v + 1 - dx]
-                        for (int dx = 0; dx < 3; ++dx)
-                            tma_load_4d(gsm + s * kWgGB + dx * 4 * kRunPlaneB, &a.g, 2 * (w.x0 + 1 - dx), w.y, zz, 0, &gfull[s]);
-                        ++k;
+                for (int zz = w.z0 - 1; ok && zz <= w.z1; ++zz, ++g) {
+                    const int sl = g % kWgRing;
+                    if (g >= kWgRing && !mbar_wait1(&empty[sl], ((g / kWgRing) - 1) & 1, a.err, 31)) {
+                        ok = false;
+                        break;
                     }
+                    mbar_arrive_expect(&full[sl], (uint32_t)L::kGroupB);
+                    for (int dy = 0; dy < 3; ++dy)
+                        tma_load_4d(smem + sl * L::kGroupB + dy * 4 * kRunPlaneB, &a.a, 2 * w.x0, w.y + dy - 1, zz, 0, &full[sl]);
+                    if (zz < w.z0 || zz >= w.z1) continue;
+                    const int s = k & 1;
+                    if (k >= 2 && !mbar_wait1(&bempty[s], ((k >> 1) - 1) & 1, a.err, 34)) {
+                        ok = false;
+                        break;
+                    }
+                    mbar_arrive_expect(&bfull[s], (uint32_t)L::kCopyB);
+                    // copy dx holds B[v + 1 - dx]
+                    for (int dx = 0; dx < 3; ++dx)
+                        tma_load_4d(bsm + s * L::kCopyB + dx * BP * kRunPlaneB, &a.b, 2 * (w.x0 + 1 - dx), w.y, zz, 0, &bfull[s]);
+                    ++k;
+                }
             }
         }
     } else if (warp == 1) {
         // the whole warp runs the loop, one lane issues; hand-overs are committed a few MMAs into the next
         // line (see k_conv3)
-        constexpr uint32_t idesc = idesc_bf16_mn(96);
+        constexpr uint32_t idesc = idesc_bf16_mn(L::kCols);
         const uint32_t on = elect_one();
         bool ok = true;
-        int g = 0, k = 0;
-        int crel = 0, cg = 0, cs = -1;  // the line before: groups to release from group cg on, its copies of G
+        int g = 0, k = 0, f = 0;                  // row groups, lines, chains begun
+        const int nu = (int)((U - blockIdx.x + gridDim.x - 1) / gridDim.x), half = nu - (nu + 1) / 3;
+        int n = 0;                               // units begun
+        int crel = 0, cg = 0, cs = -1, cf = -1;  // the line before: groups to release from group cg on, its copies of B, the set it completes
         auto commit = [&] {
             if (on && cs >= 0) {
-                mma_commit(&gempty[cs]);
+                mma_commit(&bempty[cs]);
                 for (int j = 0; j < crel; ++j) mma_commit(&empty[(cg + j) % kWgRing]);
+                if (cf >= 0) mma_commit(&sfull[cf]);
             }
             __syncwarp();
         };
@@ -572,56 +600,76 @@ __global__ void __launch_bounds__(192, 1) k_wgrad(const __grid_constant__ WgradA
             for (int i = 0; i < nz; ++i, ++k) {
                 const int s = k & 1;
                 if (i == 0) {
-                    // the first two groups of a unit may wait for slots that the last line still holds
+                    // a unit's first line may wait for slots or sums that the last line still holds
                     commit();
                     cs = -1;
                 }
+                const bool begin = BP == 2 || (i == 0 && (n == 0 || n == half));
+                const int set = f % L::kSets;
                 for (int j = i == 0 ? 0 : 2; j < 3 && ok; ++j) {
                     const int gg = g + i + j;
                     ok = mbar_wait(&full[gg % kWgRing], (gg / kWgRing) & 1, a.err, 32);
                 }
-                if (ok) ok = mbar_wait(&gfull[s], (k >> 1) & 1, a.err, 35);
+                if (ok) ok = mbar_wait(&bfull[s], (k >> 1) & 1, a.err, 35);
+                if (ok && begin && f >= L::kSets) ok = mbar_wait(&sread[set], (f / L::kSets - 1) & 1, a.err, 37);
                 if (!ok) break;
                 tc_fence_after();
-                const uint64_t b0 = sdesc(smem_u32(gsm + s * kWgGB), 128, kRunPlaneB);
-                const uint32_t acc = k > 0 ? 1u : 0u;
+                const uint64_t b0 = sdesc(smem_u32(bsm + s * L::kCopyB), 128, kRunPlaneB);
+                const uint32_t acc = begin ? 0u : 1u;
 #pragma unroll
                 for (int j = 0; j < 3; ++j) {
-                    const uint64_t a0 = sdesc(smem_u32(smem) + (uint32_t)(((g + i + j) % kWgRing) * kWgGroupB), 128, kRunPlaneB);
+                    const uint64_t a0 = sdesc(smem_u32(smem) + (uint32_t)(((g + i + j) % kWgRing) * L::kGroupB), 128, kRunPlaneB);
 #pragma unroll
                     for (int kb = 0; kb < 8; ++kb) {
-                        mma_bf16_on(on, tmem + (uint32_t)(128 * j), a0 + 16 * kb, b0 + 16 * kb, idesc, kb > 0 ? 1u : acc);
+                        mma_bf16_on(on, tmem + (uint32_t)(128 * j + 64 * set), a0 + 16 * kb, b0 + 16 * kb, idesc, kb > 0 ? 1u : acc);
                         if (j == 0 && kb == 3) commit();
                     }
                 }
                 cs = s;
                 cg = g + i;
                 crel = i < nz - 1 ? 1 : 3;
+                const bool end = BP == 2 || (i == nz - 1 && (n == half - 1 || n == nu - 1));
+                cf = end ? set : -1;
+                if (end) ++f;
             }
             g += nz + 2;
+            ++n;
         }
         commit();
         if (on) mma_commit(done);
         __syncwarp();
         mbar_wait(done, 0, a.err, 36);
-    } else {
-        // read the 3 accumulators once every MMA of the CTA has finished
-        const int q = warp & 3;
-        if (mbar_wait(done, 0, a.err, 33, 1 << 26) && q < 3) {
-            tc_fence_after();
-            float* out = a.partial + (size_t)blockIdx.x * (32 * 32 * 27);
-            const bool anz = blockIdx.x < U;
-            for (int j = 0; j < 9; ++j) {
-                const int dz = j / 3, dx = j % 3;
-                uint32_t v[32];
-                tmem_ld32(tmem + ((uint32_t)(32 * q) << 16) + (uint32_t)(128 * dz + 32 * dx), v);
-                tmem_wait_ld();
-                const int tap = 9 * dz + 3 * q + dx;  // lane 32q + ci is row (dy = q, ci)
+    } else if ((warp & 3) < 3) {
+        const int row = 32 * (warp & 3) + lane, dy = row >> 5, ch = lane;  // row (dy, a)
+        const int dz = (warp - 2) >> 2;
+        float sum[L::kCols];
 #pragma unroll
-                for (int co = 0; co < 32; ++co)
-                    out[((size_t)co * 32 + lane) * 27 + tap] = anz ? __uint_as_float(v[co]) : 0.f;
-            }
+        for (int c = 0; c < L::kCols; ++c) sum[c] = 0.f;
+        int chains = 0;
+        for (long long u = blockIdx.x; u < U; u += gridDim.x) {
+            const Unit w = unit_of(a.N, a.tiles_x, a.unit_z, u);
+            chains = BP == 2 ? chains + w.z1 - w.z0 : chains < 2 ? chains + 1 : 2;
         }
+        for (int f = 0; f < chains; ++f) {
+            const int set = f % L::kSets;
+            if (!mbar_wait(&sfull[set], (f / L::kSets) & 1, a.err, 38, 1 << 26)) break;
+            tc_fence_after();
+#pragma unroll
+            for (int c = 0; c < L::kCols; c += 16) {
+                uint32_t v[16];
+                tmem_ld16(tmem + ((uint32_t)(32 * dy) << 16) + (uint32_t)(128 * dz + 64 * set + c), v);
+                tmem_wait_ld();
+#pragma unroll
+                for (int e = 0; e < 16; ++e) sum[c + e] += __uint_as_float(v[e]);
+            }
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&sread[set]);
+        }
+        float* out = a.partial + (size_t)blockIdx.x * (27 * 256 * BP) + ch;
+#pragma unroll
+        for (int c = 0; c < L::kCols; ++c)  // column (dx, b)
+            out[((9 * dz + 3 * dy + c / (8 * BP)) * (8 * BP) + c % (8 * BP)) * 32] = sum[c];
     }
     tc_fence_before();
     __syncthreads();
@@ -632,88 +680,37 @@ __global__ void __launch_bounds__(192, 1) k_wgrad(const __grid_constant__ WgradA
     }
 }
 
-// Weight gradients of the thin layers on the CUDA cores (the first layer: 3 input channels; the
-// last: one output channel).  A block takes one x-line at a time: the line's gradient run and, plane
-// by plane, the 9 input runs (130 voxels) go to shared memory as fp32; thread t owns the real
-// weights w = t, t + blockDim, ... in the layer's [co][ci][tap] order and accumulates over the
-// line's voxels and over every line the block visits; each block writes its partial sums.
-constexpr int kThinMaxW = 16;
-
-// Staged runs are kept channel-major, xs[e][r][x] with a row pitch of 3 mod 32 words, so that the
-// 27 taps a warp reads at one x fall in 27 different banks.
-__host__ __device__ inline int thin_pitch(int N) { return (N + 2 - 3 + 31) / 32 * 32 + 3; }
-
-__global__ void k_wgrad_thin(const uint4* X, int cin, const uint4* G, int cout, int N, long long nvox,
-                             float* partial) {
-    extern __shared__ float sm[];
-    const int RUN = N + 2, RP = thin_pitch(N);
-    float* xs = sm;                // [8][9][RP]
-    float* gs = sm + 8 * 9 * RP;   // [N][cout]
-    const int total = cout * cin * 27;
-    float acc[kThinMaxW];
+// Sums of per-block partials in a fixed order (the result does not depend on scheduling).  A block takes 32
+// entries; its 8 warps add every eighth block each, 4 loads in flight, then the warps' sums are added in
+// order.  (One thread per entry over all blocks in turn waited on 148 dependent loads: 25 us.)
+__device__ __forceinline__ float partial_sum(const float* partial, int blocks, long long stride, int i, bool in) {
+    __shared__ float red[8][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    float s[4] = {0.f, 0.f, 0.f, 0.f};
+    for (int b0 = w; b0 < blocks; b0 += 32)
 #pragma unroll
-    for (int j = 0; j < kThinMaxW; ++j) acc[j] = 0.f;
-    const long long lines = (long long)N * N;
-    const int xplanes = (cin + 7) / 8;
-    for (long long l = blockIdx.x; l < lines; l += gridDim.x) {
-        const int y = (int)(l % N), z = (int)(l / N);
-        __syncthreads();
-        for (int i = threadIdx.x; i < N * cout; i += blockDim.x) {
-            const int x = i / cout, co = i % cout;
-            const long long vox = x + (long long)N * (y + (long long)N * z);
-            const uint4 u = G[(co / 8) * nvox + vox];
-            const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
-            const float2 f = unpack_bf16(w4[(co % 8) / 2]);
-            gs[i] = (co & 1) ? f.y : f.x;
-        }
-        for (int pl = 0; pl < xplanes; ++pl) {
-            __syncthreads();
-            for (int i = threadIdx.x; i < 9 * RUN; i += blockDim.x) {
-                const int r = i / RUN, xi = i % RUN;
-                const int xx = xi - 1, yy = y + r % 3 - 1, zz = z + r / 3 - 1;
-                uint4 u = make_uint4(0u, 0u, 0u, 0u);
-                if (xx >= 0 && xx < N && yy >= 0 && yy < N && zz >= 0 && zz < N)
-                    u = X[pl * nvox + xx + (long long)N * (yy + (long long)N * zz)];
-                const uint32_t w4[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    const float2 f = unpack_bf16(w4[j]);
-                    xs[((2 * j) * 9 + r) * RP + xi] = f.x;
-                    xs[((2 * j + 1) * 9 + r) * RP + xi] = f.y;
-                }
-            }
-            __syncthreads();
-#pragma unroll
-            for (int j = 0; j < kThinMaxW; ++j) {
-                const int w = threadIdx.x + j * blockDim.x;
-                if (w < total) {
-                    const int co = w / (cin * 27), ci = (w / 27) % cin, tap = w % 27;
-                    if (ci / 8 == pl) {
-                        const int r = tap / 3, dx = tap % 3;
-                        const float* xr = xs + ((ci % 8) * 9 + r) * RP + dx;
-                        float sacc = 0.f;
-                        for (int x = 0; x < N; ++x) sacc = __fmaf_rn(xr[x], gs[x * cout + co], sacc);
-                        acc[j] += sacc;
-                    }
-                }
-            }
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < kThinMaxW; ++j) {
-        const int w = threadIdx.x + j * blockDim.x;
-        if (w < total) partial[(size_t)blockIdx.x * total + w] = acc[j];
-    }
+        for (int k = 0; k < 4; ++k)
+            if (in && b0 + 8 * k < blocks) s[k] += partial[(b0 + 8 * k) * stride + i];
+    red[w][lane] = (s[0] + s[1]) + (s[2] + s[3]);
+    __syncthreads();
+    float t = 0.f;
+    for (int k = 0; k < 8; ++k) t += red[k][lane];
+    return t;
 }
-
-// Sum of per-block partials: out[i] = sum_b partial[b * stride + i] (fixed order: the result does
-// not depend on scheduling).
-__global__ void k_sum_partials(const float* partial, int blocks, int n, int stride, float* out) {
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        float s = 0.f;
-        for (int b = 0; b < blocks; ++b) s += partial[(size_t)b * stride + i];
-        out[i] = s;
-    }
+// out[i] = sum_b partial[b * stride + i]
+__global__ void __launch_bounds__(256) k_sum_partials(const float* partial, int blocks, int n, int stride, float* out) {
+    const int i = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float t = partial_sum(partial, blocks, stride, i, i < n);
+    if (threadIdx.x < 32 && i < n) out[i] = t;
+}
+// The same for k_wgrad's partial sums [t][b][a] (BC channels b, 32 channels a), into the layer's order
+// [cout][cin][27]: co = b, ci = a, tap = t, or the other way round and mirrored (`gradient_a`).
+__global__ void __launch_bounds__(256) k_sum_wgrad(const float* partial, int blocks, int BC, int cout, int cin, int gradient_a, float* out) {
+    const int n = 27 * BC * 32, i = blockIdx.x * 32 + (threadIdx.x & 31);
+    const float s = partial_sum(partial, blocks, n, i, i < n);
+    const int ca = i & 31, cb = i / 32 % BC, t = i / (32 * BC);
+    const int co = gradient_a ? ca : cb, ci = gradient_a ? cb : ca, tap = gradient_a ? 26 - t : t;
+    if (threadIdx.x < 32 && i < n && co < cout && ci < cin) out[((size_t)co * cin + ci) * 27 + tap] = s;
 }
 
 // Per-channel sums over the voxels of a planes tensor (bias gradients): block partials [block][C].
@@ -809,8 +806,19 @@ __global__ void k_absdiff_max(const float* a, const float* b, Geom g, unsigned* 
 // channel n, as pack_layer) or, with `transpose`, the image of the convolution that maps the
 // gradient of the layer's output to the gradient of its input: input channels = the layer's
 // outputs, output channels = the layer's inputs, taps mirrored (tap -> 26 - tap).
-__global__ void k_pack_w(const float* W, int cin, int cout, int cin8, int nout, int transpose, __nv_bfloat16* img) {
-    const int halves = cin8 / 2;
+struct PackJob {
+    const float* W;  // the layer's weights; its bias follows them
+    int cin, cout, cin8, nout, transpose;
+    __nv_bfloat16* img;
+    float* bias;     // forward images only: the bias padded to nout
+};
+struct PackArgs {
+    PackJob job[2 * kLayers];
+};
+__global__ void k_pack_w(const __grid_constant__ PackArgs a) {
+    const PackJob& j = a.job[blockIdx.y];
+    const int cin = j.cin, cout = j.cout, nout = j.nout;
+    const int halves = j.cin8 / 2;
     const int n_img = 27 * halves * 2 * nout * 8;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n_img; i += gridDim.x * blockDim.x) {
         const int e = i % 8, n = (i / 8) % nout, dz = 2 - (i / (8 * nout)) % 3, kc = (i / (24 * nout)) % 2;
@@ -818,17 +826,15 @@ __global__ void k_pack_w(const float* W, int cin, int cout, int cin8, int nout, 
         const int tap = 9 * dz + r;
         const int k = 16 * h + 8 * kc + e;  // input channel of the packed convolution
         float v = 0.f;
-        if (!transpose) {
-            if (n < cout && k < cin) v = W[((size_t)n * cin + k) * 27 + tap];
+        if (!j.transpose) {
+            if (n < cout && k < cin) v = j.W[((size_t)n * cin + k) * 27 + tap];
         } else {
-            if (k < cout && n < cin) v = W[((size_t)k * cin + n) * 27 + (26 - tap)];
+            if (k < cout && n < cin) v = j.W[((size_t)k * cin + n) * 27 + (26 - tap)];
         }
-        img[i] = __float2bfloat16_rn(v);
+        j.img[i] = __float2bfloat16_rn(v);
     }
-}
-__global__ void k_pack_bias(const float* b, int cout, int nout, float* out) {
-    const int i = threadIdx.x;
-    if (i < nout) out[i] = i < cout ? b[i] : 0.f;
+    if (j.bias && blockIdx.x == 0 && threadIdx.x < nout)
+        j.bias[threadIdx.x] = threadIdx.x < cout ? j.W[(size_t)cout * cin * 27 + threadIdx.x] : 0.f;
 }
 
 // Gradient of the loss L = mean over the voxels inside the shell of ((q - y) / b)^2 with respect to
@@ -863,17 +869,24 @@ __global__ void k_loss_grad(const float* q, const float* y, Geom g, float b, flo
     }
 }
 
-// Sum of squares of the gradient (for clipping by its global norm): one block.
-__global__ void k_sumsq(const float* g, long long n, float* out) {
+// Sum of squares of the gradient (for clipping by its global norm): one block, 8 loads in flight per thread.
+__global__ void __launch_bounds__(1024) k_sumsq(const float* g, long long n, float* out) {
     __shared__ float red[32];
-    float acc = 0.f;
-    for (long long i = threadIdx.x; i < n; i += blockDim.x) acc = __fmaf_rn(g[i], g[i], acc);
+    float a8[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    for (long long i = threadIdx.x; i < n; i += 8 * 1024) {
+        float v[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = i + k * 1024 < n ? g[i + k * 1024] : 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) a8[k] = __fmaf_rn(v[k], v[k], a8[k]);
+    }
+    float acc = ((a8[0] + a8[1]) + (a8[2] + a8[3])) + ((a8[4] + a8[5]) + (a8[6] + a8[7]));
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(FULL, acc, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = acc;
     __syncthreads();
     if (threadIdx.x == 0) {
         float t = 0.f;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
+        for (int w = 0; w < 32; ++w) t += red[w];
         *out = t;
     }
 }
@@ -1131,65 +1144,60 @@ static gell_status run_layers(gell_ctx* c, int sub, SurrogateState* S, int layer
 }
 static gell_status infer(gell_ctx* c, int sub, SurrogateState* S) { return run_layers(c, sub, S, kLayers); }
 
-// Shapes of the data-gradient convolution of layer l: input planes (the layer's outputs, padded to
-// 16 channels) and outputs (the layer's inputs).
+// Input planes of the data-gradient convolution of layer l (the layer's outputs, padded to 16 channels).
 static int dgrad_cin8(int l) { return kShape[l].cout <= 16 ? 2 : 4; }
-static int dgrad_nout(int) { return 32; }
 
 static gell_status repack(gell_ctx* c, SurrogateState* S) {
     TrainState* T = S->train;
+    PackArgs a{};
+    int n = 0;
     for (int l = 0; l < kLayers; ++l) {
         const LayerShape& sh = kShape[l];
-        GELL_KERNEL(c, "k_pack_w", (k_pack_w<<<64, 256, 0, c->stream>>>(T->master + T->off_w[l], sh.cin, sh.cout, sh.cin8,
-                                                                         sh.nout, 0, (__nv_bfloat16*)S->w[l])));
-        GELL_KERNEL(c, "k_pack_bias", (k_pack_bias<<<1, 32, 0, c->stream>>>(T->master + T->off_b[l], sh.cout, sh.nout, S->bias[l])));
-        if (l >= 1)
-            GELL_KERNEL(c, "k_pack_w", (k_pack_w<<<64, 256, 0, c->stream>>>(T->master + T->off_w[l], sh.cin, sh.cout,
-                                                                             dgrad_cin8(l), dgrad_nout(l), 1,
-                                                                             (__nv_bfloat16*)T->wt[l])));
+        const float* W = T->master + T->off_w[l];
+        a.job[n++] = PackJob{W, sh.cin, sh.cout, sh.cin8, sh.nout, 0, (__nv_bfloat16*)S->w[l], S->bias[l]};
+        if (l >= 1) a.job[n++] = PackJob{W, sh.cin, sh.cout, dgrad_cin8(l), kHidden, 1, (__nv_bfloat16*)T->wt[l], nullptr};
     }
+    GELL_KERNEL(c, "k_pack_w", (k_pack_w<<<dim3(16, n), 256, 0, c->stream>>>(a)));
     return GELL_OK;
 }
 
-static int thin_blocks() { return 148 * 4; }
+template <int BP>
+static gell_status launch_wgrad(gell_ctx* c, TrainState* T, const LayerShape& sh, const PlaneMaps& A, const PlaneMaps& B,
+                                bool gradient_a, float* out) {
+    using L = WgradSmem<BP>;
+    const int N = c->g.N;
+    WgradArgs a{};
+    a.a = A.all;
+    a.b = B.all;
+    a.partial = T->partial;
+    a.N = N;
+    a.tiles_x = (N + kTileM - 1) / kTileM;
+    a.err = c->dev_err;
+    int sms = 0;
+    GELL_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+    a.unit_z = unit_lines(N, sms);
+    const long long units = (long long)a.tiles_x * ((N + a.unit_z - 1) / a.unit_z) * N;
+    int grid = (int)(units < sms ? units : sms);
+    if (grid > kWgCtas) grid = kWgCtas;
+    GELL_CUDA(c, cudaFuncSetAttribute(k_wgrad<BP>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
+    GELL_KERNEL(c, BP == 2 ? "k_wgrad_thin" : "k_wgrad", (k_wgrad<BP><<<grid, kWgThreads, L::kBytes, c->stream>>>(a)));
+    const int n = 27 * 256 * BP;
+    GELL_KERNEL(c, "k_sum_partials", (k_sum_wgrad<<<n / 32, 256, 0, c->stream>>>(T->partial, grid, 8 * BP, sh.cout, sh.cin, gradient_a, out)));
+    return GELL_OK;
+}
 
-// Weight gradient of layer l into T->grad (the layer's block): tcgen05 for the 32 -> 32 layers,
-// CUDA cores for the thin first and last layers; bias gradient = per-channel sums of G.
-static gell_status wgrad_layer(gell_ctx* c, SurrogateState* S, int l, const PlaneMaps* xmap, const uint4* X,
-                               const PlaneMaps* gmap, const uint4* G, int gplanes) {
+// Weight gradient of layer l into T->grad (the layer's block); bias gradient = per-channel sums of G.
+static gell_status wgrad_layer(gell_ctx* c, SurrogateState* S, int l, const PlaneMaps& x, const PlaneMaps& g, const uint4* G) {
     TrainState* T = S->train;
     const LayerShape& sh = kShape[l];
-    const int N = c->g.N;
-    const int nw = sh.cout * sh.cin * 27;
-    if (sh.cin == kHidden && sh.cout == kHidden) {
-        WgradArgs a{};
-        a.x = xmap->all;
-        a.g = gmap->all;
-        a.partial = T->partial;
-        a.N = N;
-        a.tiles_x = (N + kTileM - 1) / kTileM;
-        a.err = c->dev_err;
-        int sms = 0;
-        GELL_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-        a.unit_z = unit_lines(N, sms);
-        const long long units = (long long)a.tiles_x * ((N + a.unit_z - 1) / a.unit_z) * N;
-        const int grid = (int)(units < sms ? units : sms);
-        GELL_CUDA(c, cudaFuncSetAttribute(k_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, kWgBytes));
-        GELL_KERNEL(c, "k_wgrad", (k_wgrad<<<grid, 192, kWgBytes, c->stream>>>(a)));
-        GELL_KERNEL(c, "k_sum_partials", (k_sum_partials<<<(nw + 255) / 256, 256, 0, c->stream>>>(T->partial, grid, nw, nw,
-                                                                                                  T->grad + T->off_w[l])));
-    } else {
-        const int smem = (8 * 9 * thin_pitch(N) + N * sh.cout) * 4;
-        GELL_CUDA(c, cudaFuncSetAttribute(k_wgrad_thin, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        GELL_KERNEL(c, "k_wgrad_thin", (k_wgrad_thin<<<thin_blocks(), 256, smem, c->stream>>>(X, sh.cin, G, sh.cout, N,
-                                                                                                c->nvox, T->partial)));
-        GELL_KERNEL(c, "k_sum_partials", (k_sum_partials<<<(nw + 255) / 256, 256, 0, c->stream>>>(
-                                              T->partial, thin_blocks(), nw, nw, T->grad + T->off_w[l])));
-    }
-    const int C = gplanes * 8;
-    GELL_KERNEL(c, "k_channel_sums", (k_channel_sums<<<thin_blocks(), 256, 0, c->stream>>>(G, gplanes, c->nvox, T->partial)));
-    GELL_KERNEL(c, "k_sum_partials", (k_sum_partials<<<1, 32, 0, c->stream>>>(T->partial, thin_blocks(), sh.cout, C,
-                                                                              T->grad + T->off_b[l])));
+    float* out = T->grad + T->off_w[l];
+    const gell_status st = l == 0           ? launch_wgrad<2>(c, T, sh, g, x, true, out)
+                           : l == kLayers - 1 ? launch_wgrad<2>(c, T, sh, x, g, false, out)
+                                              : launch_wgrad<4>(c, T, sh, x, g, false, out);
+    if (st != GELL_OK) return st;
+    const int planes = (sh.cout + 7) / 8, blocks = 148 * 4;
+    GELL_KERNEL(c, "k_channel_sums", (k_channel_sums<<<blocks, 256, 0, c->stream>>>(G, planes, c->nvox, T->partial)));
+    GELL_KERNEL(c, "k_sum_partials", (k_sum_partials<<<1, 256, 0, c->stream>>>(T->partial, blocks, sh.cout, 8 * planes, T->grad + T->off_b[l])));
     return GELL_OK;
 }
 
@@ -1240,18 +1248,18 @@ static gell_status train_pair(gell_ctx* c, int sub, SurrogateState* S, float lr,
     const int lb = 148 * 8;
     GELL_KERNEL(c, "k_loss_grad", (k_loss_grad<<<lb, 256, 0, c->stream>>>(S->ph, T->tgt, c->g, loss_unit, 1.f / (float)inner, T->gd,
                                                                           T->scal + 2)));
-    GELL_KERNEL(c, "k_sum_partials", (k_sum_partials<<<1, 32, 0, c->stream>>>(T->scal + 2, lb, 1, 1, T->scal + 1)));
+    GELL_KERNEL(c, "k_sum_partials", (k_sum_partials<<<1, 256, 0, c->stream>>>(T->scal + 2, lb, 1, 1, T->scal + 1)));
 
     // backward
-    if ((st = wgrad_layer(c, S, 9, nullptr, T->hb[4], nullptr, T->gd, 1)) != GELL_OK) return st;
+    if ((st = wgrad_layer(c, S, 9, T->mh[4], T->mgd, T->gd)) != GELL_OK) return st;
     st = launch_conv<2, 32, kLinear>(c, "k_conv3_dgrad", T->mgd, T->wt[9], T->zero_bias, T->gh, nullptr, nullptr, nullptr,
                                      nullptr, 0.f, 0.f);
     for (int k = 3; k >= 0 && st == GELL_OK; --k) {
-        if ((st = wgrad_layer(c, S, 2 * k + 2, &T->mt[k], T->tb[k], &T->mgh, T->gh, 4)) != GELL_OK) return st;
+        if ((st = wgrad_layer(c, S, 2 * k + 2, T->mt[k], T->mgh, T->gh)) != GELL_OK) return st;
         st = launch_conv<4, 32, kMask>(c, "k_conv3_dgrad", T->mgh, T->wt[2 * k + 2], T->zero_bias, T->gu, nullptr,
                                        T->tb[k], nullptr, nullptr, 0.f, 0.f);
         if (st != GELL_OK) return st;
-        if ((st = wgrad_layer(c, S, 2 * k + 1, &T->mh[k], T->hb[k], &T->mgu, T->gu, 4)) != GELL_OK) return st;
+        if ((st = wgrad_layer(c, S, 2 * k + 1, T->mh[k], T->mgu, T->gu)) != GELL_OK) return st;
         if (k > 0)
             st = launch_conv<4, 32, kResidual>(c, "k_conv3_dgrad", T->mgu, T->wt[2 * k + 1], T->zero_bias, T->gh, T->gh,
                                                nullptr, nullptr, nullptr, 0.f, 0.f);
@@ -1260,7 +1268,7 @@ static gell_status train_pair(gell_ctx* c, int sub, SurrogateState* S, float lr,
                                               nullptr, nullptr, 0.f, 0.f);
     }
     if (st != GELL_OK) return st;
-    if ((st = wgrad_layer(c, S, 0, nullptr, S->in, nullptr, T->gh, 4)) != GELL_OK) return st;
+    if ((st = wgrad_layer(c, S, 0, S->map_in, T->mgh, T->gh)) != GELL_OK) return st;
 
     // Adam on the clipped gradient, new images
     GELL_KERNEL(c, "k_sumsq", (k_sumsq<<<1, 1024, 0, c->stream>>>(T->grad, T->count, T->scal)));
@@ -1408,7 +1416,7 @@ gell_status gell_surrogate_train_init(gell_ctx* c, int sub, const float* weights
             off += kShape[l].cout;
         }
         const size_t plane = (size_t)c->nvox * 16, field = (size_t)c->nvox_p * 4;
-        T->partial_n = 148LL * 32 * 32 * 27;
+        T->partial_n = (long long)kWgCtas * kWgPart;
         bool ok = cudaMalloc(&T->master, count * 4) == cudaSuccess && cudaMalloc(&T->grad, count * 4) == cudaSuccess &&
                   cudaMalloc(&T->m, count * 4) == cudaSuccess && cudaMalloc(&T->v, count * 4) == cudaSuccess &&
                   cudaMalloc(&T->partial, T->partial_n * 4) == cudaSuccess &&
@@ -1419,7 +1427,7 @@ gell_status gell_surrogate_train_init(gell_ctx* c, int sub, const float* weights
         for (int k = 0; ok && k < 5; ++k) ok = cudaMalloc(&T->hb[k], 4 * plane) == cudaSuccess;
         for (int k = 0; ok && k < 4; ++k) ok = cudaMalloc(&T->tb[k], 4 * plane) == cudaSuccess;
         for (int l = 1; ok && l < kLayers; ++l)
-            ok = cudaMalloc(&T->wt[l], (size_t)27 * (dgrad_cin8(l) / 2) * 2 * dgrad_nout(l) * 8 * 2) == cudaSuccess;
+            ok = cudaMalloc(&T->wt[l], (size_t)27 * (dgrad_cin8(l) / 2) * 2 * kHidden * 8 * 2) == cudaSuccess;
         if (!ok) return fail(c, GELL_ERR_ALLOC, "surrogate training buffers (46 planes of 16 bytes per voxel)");
         GELL_CUDA(c, cudaMemsetAsync(T->zero_bias, 0, 32 * 4, c->stream));
         GELL_CUDA(c, cudaMemsetAsync(T->gd, 0, 2 * plane, c->stream));

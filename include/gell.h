@@ -414,8 +414,7 @@ gell_status gell_ensemble_get_batched(const gell_ensemble* ens, int* on);
  * gell_surrogate_train_pair: one pair of the running model.  The plain solver advances the field by
  * `substeps` (the target); the operator runs from the field before them; the loss is the mean of
  * ((q - target) / b)^2 inside the boundary layers.  Its gradient goes back through the ten layers:
- * data gradients on the tensor cores; weight gradients on the tensor cores for the 32 -> 32
- * layers, on the CUDA cores for the first and last. Adam (0.9, 0.999, 1e-8) takes a step of rate
+ * data and weight gradients on the tensor cores. Adam (0.9, 0.999, 1e-8) takes a step of rate
  * `lr` on the gradient clipped to global norm 1.  The field is left at the target.  *loss (if not
  * NULL) gets the loss before the step (synchronises).
  * gell_surrogate_train_read: which 0 = the master weights, 1 = the last gradient (count =
