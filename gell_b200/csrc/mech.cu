@@ -7,8 +7,9 @@
 //                 list: the first and last sorted index of every occupied bin, stamped with the
 //                 step's epoch (replaces Mech_Mesh_se_Reset/Get, :38-53, which rewrite 2*N^3 ints)
 //   k_force_move  forcekernel (:56-118) and movementkernel (:130-158) fused: one thread per cell
-//                 walks the 27 bins in the reference's order and applies the move; it reads the
-//                 sorted buffer and writes the other one, so no cell sees a moved neighbour
+//                 (few cells: k_force_warp, one warp) walks the 27 bins in the reference's order and
+//                 applies the move; it reads the sorted buffer and writes the other one, so no cell
+//                 sees a moved neighbour
 #include "mech_body.cuh"
 
 namespace gell {
@@ -25,7 +26,14 @@ __global__ void k_gather(CellsSoA s, CellsSoA d, const uint32_t* __restrict__ ke
     gather_body(s, d, keys, perm, n, bins, epoch_p, blockIdx.x);
 }
 
-__global__ void __launch_bounds__(256) k_force_move(MechArgs a) { force_move_body(a, blockIdx.x); }
+__global__ void __launch_bounds__(kForceThreads) k_force_move(MechArgs a) { force_move_body(a, blockIdx.x); }
+__global__ void __launch_bounds__(kForceThreads) k_force_warp(MechArgs a) { force_move_warp_body(a, blockIdx.x); }
+
+// A warp per cell up to here, a thread per cell beyond (us, both measured: 2,000 cells 9 against 32, 10,000 14
+// against 34, 30,000 25 against 36, 60,000 41 against 35).
+constexpr int kForceWarpCells = 48000;
+// cells per block of the force kernel that takes n cells
+int force_block(long long n) { return n <= kForceWarpCells ? kForceThreads / 32 : kForceThreads; }
 
 // Reference-shaped s/e arrays (first and last LIVE sorted index per bin, Max_Cell_num+1 / -1 when
 // empty) rebuilt from the cell list, for the parity tests.
@@ -79,8 +87,12 @@ gell_status fm_update(gell_ctx* c) {
         a.cccr = c->P.cccr;
         a.ccca = c->P.ccca;
         a.ra_ratio = c->P.ra_ratio;
+        a.ra_f = (float)a.ra_ratio;
+        a.ra_exact = (double)a.ra_f == a.ra_ratio;
+        a.sure = a.ra_ratio > 0.0 ? 1.f - 0x1p-18f : -1.f;
         a.half_dt = c->P.mechanics_dt / 2.f;
-        GELL_KERNEL(c, "k_force_move", k_force_move<<<blocks_for(n, 256), 256, 0, c->stream>>>(a));
+        const int per = force_block(n);
+        GELL_KERNEL(c, "k_force_move", (per < kForceThreads ? k_force_warp : k_force_move)<<<blocks_for(n, per), kForceThreads, 0, c->stream>>>(a));
         c->sign.swap();
         c->mesh.swap();
         c->posr.swap();
@@ -193,10 +205,15 @@ struct ForceBatch {
     BlockMap map;
     MechArgs job[kBatchMembers];
 };
-__global__ void __launch_bounds__(256) k_force_move_batch(const __grid_constant__ ForceBatch b) {
+__global__ void __launch_bounds__(kForceThreads) k_force_move_batch(const __grid_constant__ ForceBatch b) {
     int local;
     const MechArgs& j = b.job[member_of(b.map, blockIdx.x, local)];
     force_move_body(j, local);
+}
+__global__ void __launch_bounds__(kForceThreads) k_force_warp_batch(const __grid_constant__ ForceBatch b) {
+    int local;
+    const MechArgs& j = b.job[member_of(b.map, blockIdx.x, local)];
+    force_move_warp_body(j, local);
 }
 
 // the uptake map's arguments (lod.cu's PreArgs for at most kBatchSub substrates) and the cells
@@ -323,6 +340,10 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
         }
         GELL_KERNEL(c0, "k_gather_batch", k_gather_batch<<<gblocks, 256, 0, st>>>(gb));
 
+        long long cells = 0;
+        for (gell_ctx* c : fm) cells += c->n;
+        const int per = force_block(cells);
+        for (int i = 0; i < nf; ++i) blocks[i] = blocks_for(fm[i]->n, per);
         ForceBatch fb{};
         const int fblocks = fill_map(fb.map, blocks);
         for (int i = 0; i < nf; ++i) {
@@ -338,6 +359,9 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
             a.cccr = c->P.cccr;
             a.ccca = c->P.ccca;
             a.ra_ratio = c->P.ra_ratio;
+        a.ra_f = (float)a.ra_ratio;
+        a.ra_exact = (double)a.ra_f == a.ra_ratio;
+        a.sure = a.ra_ratio > 0.0 ? 1.f - 0x1p-18f : -1.f;
             a.half_dt = c->P.mechanics_dt / 2.f;
             c->sign.swap();
             c->mesh.swap();
@@ -345,7 +369,8 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
             c->force.swap();
             c->oldf.swap();
         }
-        GELL_KERNEL(c0, "k_force_move_batch", k_force_move_batch<<<fblocks, 256, 0, st>>>(fb));
+        GELL_KERNEL(c0, "k_force_move_batch",
+                    (per < kForceThreads ? k_force_warp_batch : k_force_move_batch)<<<fblocks, kForceThreads, 0, st>>>(fb));
     }
     for (gell_ctx* c : ms) {
         c->sorted_valid = true;
