@@ -2,7 +2,8 @@
 //
 //   k_keys        Morton key + 1 per cell, 0 (and sign = false) for a cell outside the grid;
 //                 mesh_idx of the cells inside (updateCellMeshIdx, :22-36)
-//   radix_sort    stable sort of (key, index) (thrust::sort_by_key, :190), sort.cu
+//   radix_sort    stable sort of (key, index) (thrust::sort_by_key, :190), sort.cu; up to 6,144 cells
+//                 k_sort_one does keys and sort in one CTA
 //   k_gather      every cell field moved to its sorted slot in the other buffer, and the cell
 //                 list: the first and last sorted index of every occupied bin, stamped with the
 //                 step's epoch (replaces Mech_Mesh_se_Reset/Get, :38-53, which rewrite 2*N^3 ints)
@@ -19,6 +20,8 @@ namespace {
 __global__ void k_keys(CellsSoA c, int n, Geom g, uint32_t* __restrict__ keys, int* __restrict__ epoch) {
     keys_body(c, n, g, keys, epoch, blockIdx.x);
 }
+
+__global__ void __launch_bounds__(kOneThreads, 1) k_sort_one(const __grid_constant__ OneJob a) { sort_one_body(a); }
 
 __global__ void k_gather(CellsSoA s, CellsSoA d, const uint32_t* __restrict__ keys,
                          const uint32_t* __restrict__ perm, int n, int4* __restrict__ bins,
@@ -65,13 +68,23 @@ static int key_bits(int N) {
     return bits;
 }
 
+static OneJob one_job(gell_ctx* c) {
+    return OneJob{c->cur(), c->g, c->sort.keys[0], c->sort.vals[0], c->dev_epoch, c->n, key_bits(c->g.N)};
+}
+
 gell_status fm_update(gell_ctx* c) {
     const int n = c->n;
     if (n > 0) {
-        GELL_KERNEL(c, "k_keys", k_keys<<<blocks_for(n, 256), 256, 0, c->stream>>>(c->cur(), n, c->g, c->sort.keys[0],
-                                                                                c->dev_epoch));
-        gell_status st = radix_sort(c, n, key_bits(c->g.N), true);
-        if (st != GELL_OK) return st;
+        if (n <= kOneCells) {
+            GELL_CUDA(c, cudaFuncSetAttribute(k_sort_one, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneSmem));
+            GELL_KERNEL(c, "k_sort_one", k_sort_one<<<1, kOneThreads, kOneSmem, c->stream>>>(one_job(c)));
+            c->sort.which = 0;
+        } else {
+            GELL_KERNEL(c, "k_keys", k_keys<<<blocks_for(n, 256), 256, 0, c->stream>>>(c->cur(), n, c->g, c->sort.keys[0],
+                                                                                    c->dev_epoch));
+            gell_status st = radix_sort(c, n, key_bits(c->g.N), true);
+            if (st != GELL_OK) return st;
+        }
         const int w = c->sort.which;
         GELL_KERNEL(c, "k_gather", k_gather<<<blocks_for(n, 256), 256, 0, c->stream>>>(c->cur(), c->alt(), c->sort.keys[w], c->sort.vals[w], n,
                                                               c->bins, c->dev_epoch));
@@ -183,6 +196,13 @@ __global__ void __launch_bounds__(kSortThreads) k_scatter_batch(const __grid_con
                  local);
 }
 
+struct OneBatch {
+    OneJob job[kBatchMembers];
+};
+__global__ void __launch_bounds__(kOneThreads, 1) k_sort_one_batch(const __grid_constant__ OneBatch b) {
+    sort_one_body(b.job[blockIdx.x]);
+}
+
 struct GatherJob {
     CellsSoA s, d;
     const uint32_t* keys;
@@ -283,24 +303,37 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
         if (c->n > 0) fm.push_back(c);
     if (!fm.empty()) {
         const int nf = (int)fm.size();
-        std::vector<int> blocks(nf);
-        for (int i = 0; i < nf; ++i) blocks[i] = blocks_for(fm[i]->n, 256);
-
-        KeysBatch kb{};
-        const int kblocks = fill_map(kb.map, blocks);
+        std::vector<int> blocks(nf), large;
+        OneBatch ob{};
+        int small = 0;
         for (int i = 0; i < nf; ++i) {
-            gell_ctx* c = fm[i];
-            kb.job[i] = KeysJob{c->cur(), c->sort.keys[0], c->dev_epoch, c->g, c->n};
+            blocks[i] = blocks_for(fm[i]->n, 256);
+            if (fm[i]->n <= kOneCells) ob.job[small++] = one_job(fm[i]);
+            else large.push_back(i);
         }
-        GELL_KERNEL(c0, "k_keys_batch", k_keys_batch<<<kblocks, 256, 0, st>>>(kb));
+        if (small > 0) {
+            GELL_CUDA(c0, cudaFuncSetAttribute(k_sort_one_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneSmem));
+            GELL_KERNEL(c0, "k_sort_one_batch", k_sort_one_batch<<<small, kOneThreads, kOneSmem, st>>>(ob));
+        }
+        if (!large.empty()) {
+            KeysBatch kb{};
+            std::vector<int> kb_blocks;
+            for (size_t k = 0; k < large.size(); ++k) {
+                gell_ctx* c = fm[large[k]];
+                kb_blocks.push_back(blocks[large[k]]);
+                kb.job[k] = KeysJob{c->cur(), c->sort.keys[0], c->dev_epoch, c->g, c->n};
+            }
+            const int kblocks = fill_map(kb.map, kb_blocks);
+            GELL_KERNEL(c0, "k_keys_batch", k_keys_batch<<<kblocks, 256, 0, st>>>(kb));
+        }
 
-        // the sort: each member's own digit width and pass count (radix_sort's rule)
-        std::vector<int> passes(nf), dbits(nf), in(nf, 0), iota(nf, 1);
+        // the sort of the others: each member's own digit width and pass count (radix_sort's rule)
+        std::vector<int> passes(nf, 0), dbits(nf, 0), in(nf, 0), iota(nf, 1);
         int maxp = 0;
-        for (int i = 0; i < nf; ++i) {
-            const int bits = key_bits(fm[i]->g.N);
-            passes[i] = (bits + 7) / 8 < 1 ? 1 : (bits + 7) / 8;
-            dbits[i] = (bits + passes[i] - 1) / passes[i];
+        for (int i : large) {
+            const SortPlan plan = sort_plan(key_bits(fm[i]->g.N));
+            passes[i] = plan.passes;
+            dbits[i] = plan.bits;
             maxp = passes[i] > maxp ? passes[i] : maxp;
         }
         for (int p = 0; p < maxp; ++p) {
@@ -315,13 +348,14 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
                 sb.job[who.size()] = SortJob{S.keys[in[i]], S.vals[in[i]], S.keys[in[i] ^ 1], S.vals[in[i] ^ 1], S.hist,
                                              c->n, nb, p * dbits[i], R, iota[i]};
                 tiles.push_back(nb);
-                digits.push_back(R);
+                digits.push_back(nb > kSortScanTiles ? R : 0);
                 who.push_back(i);
             }
             const int ntiles = fill_map(sb.tiles, tiles);
             const int ndigits = fill_map(sb.digits, digits);
             GELL_KERNEL(c0, "k_hist_batch", k_hist_batch<<<ntiles, kSortThreads, 0, st>>>(sb));
-            GELL_KERNEL(c0, "k_digit_scan_batch", k_digit_scan_batch<<<ndigits, kSortThreads, 0, st>>>(sb));
+            if (ndigits > 0)
+                GELL_KERNEL(c0, "k_digit_scan_batch", k_digit_scan_batch<<<ndigits, kSortThreads, 0, st>>>(sb));
             GELL_KERNEL(c0, "k_scatter_batch", k_scatter_batch<<<ntiles, kSortThreads, 0, st>>>(sb));
             for (int i : who) {
                 in[i] ^= 1;

@@ -310,9 +310,23 @@ __device__ __forceinline__ void force_move_warp_body(const MechArgs& a, int blk)
 
 // ------------------------------------------------------------------ radix sort (sort.cu)
 
-constexpr int kSortThreads = 256;
-constexpr int kSortItems = 16;
+constexpr int kSortThreads = 512;
+constexpr int kSortWarps = kSortThreads / 32;
+constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;  // 4096
+constexpr int kSortBits = 10;                         // bits of a digit, at most
+constexpr int kSortDigits = 1 << kSortBits;
+// Up to this many tiles the scatter adds the other tiles' counts itself (a row of at most 32 words a digit).
+constexpr int kSortScanTiles = 32;
+
+struct SortPlan {
+    int passes, bits;
+};
+// As few passes as digits of 10 bits allow, in equal digits (4 passes of 7 bits to 3 of 9 at 400^3).
+__host__ __device__ __forceinline__ SortPlan sort_plan(int bits) {
+    const int passes = bits <= kSortBits ? 1 : (bits + kSortBits - 1) / kSortBits;
+    return SortPlan{passes, (bits + passes - 1) / passes};
+}
 
 __device__ __forceinline__ unsigned lanemask_lt() {
     unsigned m;
@@ -320,18 +334,37 @@ __device__ __forceinline__ unsigned lanemask_lt() {
     return m;
 }
 
+// The valid lanes whose digit (`bits` bits) is this lane's, by one vote a bit: the match instruction takes the
+// lanes' values one after the other (k_scatter at 1M cells 20.8 -> 19.2 us).
+__device__ __forceinline__ unsigned digit_peers(uint32_t dig, int bits, bool valid) {
+    unsigned peers = __ballot_sync(FULL, valid);
+#pragma unroll
+    for (int b = 0; b < kSortBits; ++b) {
+        if (b >= bits) break;
+        const unsigned one = __ballot_sync(FULL, dig >> b & 1u);
+        peers &= dig >> b & 1u ? one : ~one;
+    }
+    return peers;
+}
+
+// Every thread's keys are requested before the first is counted: with a request between two counts a tile
+// waited for memory once per item (a launch at 1M cells, with its start: 10.6 -> 7.1 us).
 __device__ __forceinline__ void hist_body(const uint32_t* __restrict__ keys, int n, int shift, int R,
                                           uint32_t* __restrict__ hist, int nb, int blk) {
-    __shared__ uint32_t h[256];
+    __shared__ uint32_t h[kSortDigits];
+    const long long base = (long long)blk * kSortTile;
+    uint32_t key[kSortItems];
+#pragma unroll
+    for (int k = 0; k < kSortItems; ++k) {
+        const long long i = base + k * kSortThreads + threadIdx.x;
+        key[k] = i < n ? keys[i] : 0u;
+    }
     for (int d = threadIdx.x; d < R; d += kSortThreads) h[d] = 0;
     __syncthreads();
-    const long long base = (long long)blk * kSortTile;
     const uint32_t mask = (uint32_t)R - 1u;
-#pragma unroll 4
-    for (int k = 0; k < kSortItems; ++k) {
-        long long i = base + k * kSortThreads + threadIdx.x;
-        if (i < n) atomicAdd(&h[(keys[i] >> shift) & mask], 1u);
-    }
+#pragma unroll
+    for (int k = 0; k < kSortItems; ++k)
+        if (base + k * kSortThreads + threadIdx.x < n) atomicAdd(&h[(key[k] >> shift) & mask], 1u);
     __syncthreads();
     for (int d = threadIdx.x; d < R; d += kSortThreads) hist[(long long)d * nb + blk] = h[d];
 }
@@ -366,77 +399,223 @@ __device__ __forceinline__ void digit_scan_body(uint32_t* __restrict__ hist, int
     if (threadIdx.x == kSortThreads - 1) totals[blk] = run;
 }
 
+// The tile's keys and payloads are requested at the start, for the same reason as in hist_body (a
+// launch at 1M cells 23.2 -> 19.2 us; what bounds it is the 4-byte scatter).
 __device__ __forceinline__ void scatter_body(const uint32_t* __restrict__ kin, const uint32_t* __restrict__ vin,
                                              uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int n, int shift,
                                              int R, const uint32_t* __restrict__ offs, int nb,
                                              const uint32_t* __restrict__ totals, int iota, int blk) {
-    __shared__ uint32_t wcnt[kSortThreads / 32][256];
-    __shared__ uint32_t gbase[256];
+    __shared__ uint16_t wcnt[kSortWarps][kSortDigits];
+    __shared__ uint32_t gbase[kSortDigits];
+    __shared__ uint32_t ws[kSortWarps];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (int i = threadIdx.x; i < (kSortThreads / 32) * 256; i += kSortThreads) (&wcnt[0][0])[i] = 0;
-    if (w == 0) {
-        // exclusive prefix of the digit totals: lane l sums digits 8l .. 8l+7 (R <= 256)
-        uint32_t t[8], s = 0;
+    const long long base = (long long)blk * kSortTile + w * (kSortTile / kSortWarps);
+    uint32_t key[kSortItems], val[kSortItems], loc[kSortItems];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int d = 8 * lane + k;
-            t[k] = d < R ? totals[d] : 0u;
-            s += t[k];
+    for (int k = 0; k < kSortItems; ++k) {
+        const long long i = base + k * 32 + lane;
+        key[k] = i < n ? kin[i] : 0u;
+        val[k] = iota || i >= n ? (uint32_t)i : vin[i];
+    }
+    for (int i = lane; i < R / 2; i += 32) reinterpret_cast<uint32_t*>(wcnt[w])[i] = 0;
+    {
+        // this tile's first slot of each digit: thread t takes digits 2t and 2t + 1
+        uint32_t tot[2], off[2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int d = 2 * threadIdx.x + e;
+            tot[e] = off[e] = 0;
+            if (d >= R) continue;
+            const uint32_t* row = offs + (long long)d * nb;
+            if (nb <= kSortScanTiles) {
+                for (int b = 0; b < nb; ++b) {
+                    const uint32_t v = row[b];
+                    tot[e] += v;
+                    off[e] += b < blk ? v : 0u;
+                }
+            } else {
+                tot[e] = totals[d];
+                off[e] = row[blk];
+            }
         }
+        const uint32_t s = tot[0] + tot[1];
         uint32_t x = s;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(FULL, x, o);
             if (lane >= o) x += y;
         }
+        if (lane == 31) ws[w] = x;
+        __syncthreads();
         uint32_t run = x - s;
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            const int d = 8 * lane + k;
-            if (d < R) gbase[d] = run;
-            run += t[k];
+        for (int j = 0; j < w; ++j) run += ws[j];
+        const int d = 2 * threadIdx.x;
+        if (d < R) {
+            gbase[d] = run + off[0];
+            gbase[d + 1] = run + tot[0] + off[1];
         }
     }
-    __syncthreads();
-    for (int d = threadIdx.x; d < R; d += kSortThreads) gbase[d] += offs[(long long)d * nb + blk];
-    __syncthreads();
     const uint32_t mask = (uint32_t)R - 1u;
-    const long long base = (long long)blk * kSortTile + w * (kSortTile / (kSortThreads / 32));
-    uint32_t key[kSortItems], loc[kSortItems];
     const unsigned lt = lanemask_lt();
+    const int bits = __popc(mask);
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
-        const long long i = base + k * 32 + lane;
-        const bool valid = i < n;
-        key[k] = valid ? kin[i] : 0u;
+        const bool valid = base + k * 32 + lane < n;
         const uint32_t dig = (key[k] >> shift) & mask;
-        const unsigned peers = __match_any_sync(FULL, valid ? dig : 0xffffffffu);
-        const uint32_t before = wcnt[w][dig & 255];
+        const unsigned peers = digit_peers(dig, bits, valid);
+        const uint32_t before = wcnt[w][dig];
         loc[k] = before + __popc(peers & lt);
         __syncwarp();
-        if (valid && (peers & lt) == 0) wcnt[w][dig] = before + __popc(peers);
+        if (valid && (peers & lt) == 0) wcnt[w][dig] = (uint16_t)(before + __popc(peers));
         __syncwarp();
     }
     __syncthreads();
     for (int d = threadIdx.x; d < R; d += kSortThreads) {
         uint32_t run = 0;
 #pragma unroll
-        for (int ww = 0; ww < kSortThreads / 32; ++ww) {
-            uint32_t c = wcnt[ww][d];
-            wcnt[ww][d] = run;
+        for (int ww = 0; ww < kSortWarps; ++ww) {
+            const uint32_t c = wcnt[ww][d];
+            wcnt[ww][d] = (uint16_t)run;
             run += c;
         }
     }
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
-        const long long i = base + k * 32 + lane;
-        if (i < n) {
+        if (base + k * 32 + lane < n) {
             const uint32_t dig = (key[k] >> shift) & mask;
             const uint32_t pos = gbase[dig] + wcnt[w][dig] + loc[k];
             kout[pos] = key[k];
-            vout[pos] = iota ? (uint32_t)i : vin[i];
+            vout[pos] = val[k];
         }
+    }
+}
+
+// Keys and their sort for at most kOneCells cells, by one CTA that keeps keys and payloads in registers and
+// passes them through shared memory: one launch where keys and passes of their own are 5 to 7, each of which
+// takes longer to start than to sort this many.  What bounds it is the one SM's shared memory (~1,500 cycles
+// per 1,024 cells and pass), hence the line: 2,000 cells 20 us against 42 (sums of launches with their
+// starts, ~4.5 us each), 5,000 25 against 46, but 10,000 38 against 46, whose starts overlap.  The order of
+// elements is that of the tiles: chunk w of warp w, round k, lane.
+constexpr int kOneCells = 6144;
+constexpr int kOneThreads = 1024;
+constexpr int kOneRounds = kOneCells / kOneThreads;
+constexpr int kOneBits = 8;
+constexpr int kOneSmem = kOneCells * 6 + 32 * 256 * 2 + (4 * 256 + 8) * 4;
+struct OneJob {
+    CellsSoA c;
+    Geom g;
+    uint32_t *keys, *vals;
+    int* epoch;
+    int n, bits;
+};
+__device__ __forceinline__ void sort_one_body(const OneJob& a) {
+    extern __shared__ __align__(16) uint8_t one_smem[];
+    uint32_t* sk = reinterpret_cast<uint32_t*>(one_smem);
+    uint32_t* part = sk + kOneCells;                                // [4][256]
+    uint32_t* ws = part + 4 * 256;                                  // [8]
+    uint16_t* sv = reinterpret_cast<uint16_t*>(ws + 8);             // [kOneCells]
+    uint16_t* cnt = sv + kOneCells;                                 // [32][256]
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    if (t == 0) *a.epoch += 1;
+    const int n = a.n, rounds = (n + kOneThreads - 1) / kOneThreads;
+    const int first = w * rounds * 32 + lane;
+    uint32_t key[kOneRounds], vl[kOneRounds];  // payload, and its rank within warp and digit in the upper half
+#pragma unroll
+    for (int k = 0; k < kOneRounds; ++k) {
+        const int i = first + 32 * k;
+        key[k] = 0u;
+        vl[k] = (uint32_t)i;
+        if (k >= rounds || i >= n) continue;
+        const float4 pr = a.c.posr[i];
+        const int3 b = find_bin(pr.x, pr.y, pr.z, a.g.len);
+        if (!inside(b.x, b.y, b.z, a.g.N)) {
+            a.c.sign[i] = 0;
+        } else {
+            key[k] = morton3(b.x, b.y, b.z) + 1u;
+            a.c.mesh[i] = b.x + b.y * a.g.N + b.z * a.g.N * a.g.N;
+        }
+    }
+    const int passes = a.bits <= kOneBits ? 1 : (a.bits + kOneBits - 1) / kOneBits;
+    const int bits = (a.bits + passes - 1) / passes;
+    const uint32_t mask = (1u << bits) - 1u;
+    const unsigned lt = lanemask_lt();
+    for (int p = 0; p < passes; ++p) {
+        const int shift = p * bits;
+        for (int i = t; i < 32 * 256 / 2; i += kOneThreads) reinterpret_cast<uint32_t*>(cnt)[i] = 0;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kOneRounds; ++k) {
+            if (k >= rounds) break;
+            const bool valid = first + 32 * k < n;
+            const uint32_t dig = (key[k] >> shift) & mask;
+            const unsigned peers = digit_peers(dig, bits, valid);
+            const uint32_t before = cnt[w * 256 + dig];
+            vl[k] = (vl[k] & 0xffffu) | (before + __popc(peers & lt)) << 16;
+            __syncwarp();
+            if (valid && (peers & lt) == 0) cnt[w * 256 + dig] = (uint16_t)(before + __popc(peers));
+            __syncwarp();
+        }
+        __syncthreads();
+        {
+            // counts of 8 warps each, then of the quarters and digits
+            const int d = t & 255, q = t >> 8;
+            uint32_t run = 0;
+#pragma unroll
+            for (int ww = 8 * q; ww < 8 * q + 8; ++ww) {
+                const uint32_t c = cnt[ww * 256 + d];
+                cnt[ww * 256 + d] = (uint16_t)run;
+                run += c;
+            }
+            part[t] = run;
+        }
+        __syncthreads();
+        uint32_t s = 0, x = 0;
+        if (t < 256) {
+            s = part[t] + part[256 + t] + part[512 + t] + part[768 + t];
+            x = s;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, x, o);
+                if (lane >= o) x += y;
+            }
+            if (lane == 31) ws[w] = x;
+        }
+        __syncthreads();
+        if (t < 256) {
+            uint32_t run = x - s;
+            for (int j = 0; j < w; ++j) run += ws[j];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t c = part[256 * q + t];
+                part[256 * q + t] = run;
+                run += c;
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kOneRounds; ++k) {
+            if (k >= rounds || first + 32 * k >= n) continue;
+            const uint32_t dig = (key[k] >> shift) & mask;
+            const uint32_t pos = part[256 * (w >> 3) + dig] + cnt[w * 256 + dig] + (vl[k] >> 16);
+            sk[pos] = key[k];
+            sv[pos] = (uint16_t)vl[k];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kOneRounds; ++k) {
+            const int i = first + 32 * k;
+            if (k >= rounds || i >= n) continue;
+            key[k] = sk[i];
+            vl[k] = sv[i];
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kOneRounds; ++k) {
+        const int i = first + 32 * k;
+        if (k >= rounds || i >= n) continue;
+        a.keys[i] = key[k];
+        a.vals[i] = vl[k];
     }
 }
 

@@ -6,11 +6,12 @@
 // reference's -1), and only the bits a key of this grid can set are sorted.  Payloads are cell
 // indices; the cell records themselves move once, in the gather that follows (mech.cu).
 //
-// One pass per digit of d <= 8 bits: k_hist (per-tile digit counts), k_scan_hist (one CTA, exclusive
-// scan of the digit-major count table), k_scatter (stable rank inside the tile with warp match,
-// then scatter).  A tile is 8 warps x 16 items; item k of lane l of warp w is tile element
-// w*512 + k*32 + l, so processing k in order and lanes in order visits the tile in input order,
-// which is what makes the ranks, and the sort, stable.
+// One pass per digit of d <= 10 bits: k_hist (per-tile digit counts), k_digit_scan (a CTA per digit,
+// exclusive scan of its row of the digit-major count table; left out for up to 32 tiles), k_scatter
+// (stable rank inside the tile with warp match, then scatter).  A tile is 16 warps x 8 items; item k of
+// lane l of warp w is tile element w*256 + k*32 + l, so processing k in order and lanes in order visits
+// the tile in input order, which is what makes the ranks, and the sort, stable.  Up to 6,144 cells one
+// CTA does it all (k_sort_one, with the keys; mech.cu).
 #include "mech_body.cuh"
 
 namespace gell {
@@ -93,7 +94,7 @@ __global__ void __launch_bounds__(kSortThreads) k_tile_sum(const uint32_t* __res
 
 __global__ void __launch_bounds__(kSortThreads) k_tile_scan(const uint32_t* __restrict__ in, uint32_t* __restrict__ out, int n,
                                                         const uint32_t* __restrict__ offs) {
-    // thread t owns elements base + t*16 .. +15 (contiguous), so a thread-serial scan inside
+    // thread t owns elements base + t*8 .. +7 (contiguous), so a thread-serial scan inside
     // plus a block scan over threads gives the tile's exclusive scan in order
     __shared__ uint32_t ws[kSortThreads / 32];
     const long long base = (long long)blockIdx.x * kSortTile + (long long)threadIdx.x * kSortItems;
@@ -127,8 +128,8 @@ __global__ void __launch_bounds__(kSortThreads) k_tile_scan(const uint32_t* __re
 
 }  // namespace
 
-// digit-major count table, then the 256 digit totals
-size_t sort_hist_entries(int cap) { return (size_t)256 * ((cap + kSortTile - 1) / kSortTile) + 256 + 64; }
+// digit-major count table, then the digit totals
+size_t sort_hist_entries(int cap) { return (size_t)kSortDigits * ((cap + kSortTile - 1) / kSortTile) + kSortDigits + 64; }
 
 gell_status radix_sort(gell_ctx* c, int n, int bits, bool vals_are_iota) {
     SortScratch& S = c->sort;
@@ -138,16 +139,16 @@ gell_status radix_sort(gell_ctx* c, int n, int bits, bool vals_are_iota) {
         return GELL_OK;
     }
     const int nb = (n + kSortTile - 1) / kSortTile;
-    int passes = (bits + 7) / 8;
-    if (passes < 1) passes = 1;
-    const int d = (bits + passes - 1) / passes;
+    const SortPlan plan = sort_plan(bits);
+    const int passes = plan.passes, d = plan.bits;
     const int R = 1 << d;
     bool iota = vals_are_iota;
     for (int p = 0; p < passes; ++p) {
         const int shift = p * d;
         GELL_KERNEL(c, "k_hist", k_hist<<<nb, kSortThreads, 0, c->stream>>>(S.keys[in], n, shift, R, S.hist, nb));
         uint32_t* totals = S.hist + (size_t)R * nb;
-        GELL_KERNEL(c, "k_digit_scan", k_digit_scan<<<R, kSortThreads, 0, c->stream>>>(S.hist, nb, totals));
+        if (nb > kSortScanTiles)
+            GELL_KERNEL(c, "k_digit_scan", k_digit_scan<<<R, kSortThreads, 0, c->stream>>>(S.hist, nb, totals));
         GELL_KERNEL(c, "k_scatter", k_scatter<<<nb, kSortThreads, 0, c->stream>>>(S.keys[in], S.vals[in], S.keys[in ^ 1], S.vals[in ^ 1], n, shift,
                                                    R, S.hist, nb, totals, iota ? 1 : 0));
         iota = false;
