@@ -251,7 +251,8 @@ static void free_all(gell_ctx* c) {
         if (g.exec) cudaGraphExecDestroy(g.exec);
     surrogate_free(c);
     for (auto& s : c->subs) { f(s.p); f(s.rate); f(s.EF); f(s.FRS); f(s.line_flag); f(s.line_list); f(s.line_count); }
-    f(c->xorwow); f(c->flags); f(c->scan_tmp); f(c->dev_count); f(c->dev_err);
+    f(c->xorwow); f(c->flags); f(c->counts); f(c->dev_err);
+    if (c->total) cudaFreeHost(c->total);
     f(c->staging);
     for (auto& p : c->prof) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     for (auto e : c->ev_pool) cudaEventDestroy(e);
@@ -330,12 +331,12 @@ gell_status gell_create(const gell_params* params, gell_ctx** out) {
     A((void**)&c->sort.hist, sort_hist_entries(c->cap) * 4);
     A((void**)&c->bins, (size_t)c->nvox * sizeof(int4));
     A((void**)&c->dev_epoch, sizeof(int));
-    A((void**)&c->flags, (cap + 1) * 4);
-    A((void**)&c->scan_tmp, ((cap + 4095) / 4096 + 64) * 4 * 2);
-    A((void**)&c->dev_count, 64);
+    A((void**)&c->flags, cap);
+    A((void**)&c->counts, ((cap + 255) / 256) * 4);
     A((void**)&c->dev_err, 64);
     A((void**)&c->staging, cap * sizeof(gell_cell));
     if (P.rng_mode == GELL_RNG_XORWOW) A((void**)&c->xorwow, cap * sizeof(curandState));
+    if (st == GELL_OK && cudaHostAlloc((void**)&c->total, 64, cudaHostAllocDefault) != cudaSuccess) st = GELL_ERR_CUDA;
     if (st != GELL_OK) {
         free_all(c);
         delete c;

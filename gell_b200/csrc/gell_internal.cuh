@@ -145,9 +145,9 @@ struct gell_ctx {
     // PD
     curandState* xorwow = nullptr;
     uint32_t bio_step = 0;
-    uint32_t* flags = nullptr;     // cap + 1
-    uint32_t* scan_tmp = nullptr;  // block sums
-    int* dev_count = nullptr;      // device scalars for counts
+    uint8_t* flags = nullptr;      // cap: cells that divide
+    uint32_t* counts = nullptr;    // per 256 or 1,024 cells: how many divide or stay (pd.cu)
+    int* total = nullptr;          // pinned host word: their sum, written by the kernel that uses them
     int* dev_err = nullptr;        // device error word (bounded waits)
 
     gell_cell* staging = nullptr;  // cap AoS records
@@ -221,6 +221,26 @@ void prof_end(gell_ctx* c, int slot);
         (ctx)->launches++;                              \
         GELL_LAUNCH(ctx, name);                         \
     } while (0)
+
+// A launch whose CTAs may start while the kernel before it on the stream drains: such a kernel begins with
+// grid_dep_wait(), which returns when that kernel's results are there, and lets the next one start with
+// grid_dep_launch().
+template <class K, class... A>
+void launch_dependent(K kern, int grid, int block, size_t smem, cudaStream_t st, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, args...);
+}
+__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // ------------------------------------------------------------------ device helpers
 
@@ -298,8 +318,6 @@ gell_status cells_end(gell_ctx* c, gell_status st);
 gell_status birth(gell_ctx* c, int* n_out);
 gell_status death(gell_ctx* c, int* n_out);
 gell_status init_xorwow(gell_ctx* c);
-// exclusive scan of flags[0..n) into out[0..n) and the total into *total_dev
-gell_status scan_u32(gell_ctx* c, const uint32_t* in, uint32_t* out, int n, int* total_dev);
 // stable LSD radix sort of (keys, vals) over the low `bits` bits; result in c->sort.which
 gell_status radix_sort(gell_ctx* c, int n, int bits, bool vals_are_iota);
 gell_status dump_se(gell_ctx* c, int* host_out);

@@ -585,9 +585,6 @@ __global__ void __launch_bounds__(64 * kMaxComputeWarps, 1) k_sweep(const __grid
 // so that the y sweep reads its columns 4 at a time as well.
 constexpr int kPlaneMaxN = 224;  // 7 x 7 boxes of 4 KB
 
-__device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-
 struct LineCtx {
     const float* E;    // shared: E[j], 0 at the line's ends
     const float4* FR;  // shared: (-F, R, -s, L), identities (-1, 1, 0, 0) at the ends
@@ -1718,23 +1715,6 @@ static bool ring_by_default(const gell_ctx* c, int ns) {
     const int Na = (N + 31) & ~31;
     const int fixed = 1024 + align128(ns * Na * 4) + 2 * 8 * 32 * 8;
     return (227 * 1024 - fixed) / (B * kSlotFloats * 4) < 4;
-}
-
-// A launch whose CTAs may start while the kernel before it on the stream drains (the kernel itself
-// waits for that kernel's results).
-template <class K, class... A>
-static void launch_dependent(K kern, int grid, int block, size_t smem, cudaStream_t st, const A&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3((unsigned)block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 // The plane sweeps serve every grid whose plane fits in one CTA's shared memory (N <= 224), unless
