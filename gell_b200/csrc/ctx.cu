@@ -42,6 +42,8 @@ constexpr int kRecWords = sizeof(gell_cell) / 4;  // 18
 constexpr int kRecBlock = 256;
 
 __global__ void __launch_bounds__(kRecBlock) k_import(const gell_cell* __restrict__ in, CellsSoA o, int n, Geom g) {
+    grid_dep_wait();
+    grid_dep_launch();
     __shared__ __align__(16) uint32_t w[kRecBlock * kRecWords];
     const long long i0 = (long long)blockIdx.x * kRecBlock;
     const int m = n - i0 < kRecBlock ? (int)(n - i0) : kRecBlock, words = m * kRecWords;
@@ -71,6 +73,8 @@ __global__ void __launch_bounds__(kRecBlock) k_import(const gell_cell* __restric
 }
 
 __global__ void __launch_bounds__(kRecBlock) k_export(CellsSoA s, gell_cell* __restrict__ out, int n) {
+    grid_dep_wait();
+    grid_dep_launch();
     __shared__ __align__(16) uint32_t w[kRecBlock * kRecWords];
     const long long i0 = (long long)blockIdx.x * kRecBlock;
     const int m = n - i0 < kRecBlock ? (int)(n - i0) : kRecBlock, words = m * kRecWords;
@@ -104,6 +108,8 @@ __global__ void __launch_bounds__(kRecBlock) k_export(CellsSoA s, gell_cell* __r
 // element with 64-bit division and remainder by N was bound by those: 2.5 TB/s at 400^3, 207 -> 89 us.)
 __global__ void __launch_bounds__(256) k_field_copy(const float* __restrict__ in, int pin, float* __restrict__ out,
                                                     int pout, int N, long long lines) {
+    grid_dep_wait();
+    grid_dep_launch();
     if (pin == pout && ((((uintptr_t)in) | ((uintptr_t)out)) & 15) == 0) {
         const long long n4 = lines * pin / 4, step = (long long)gridDim.x * 256;  // pin = P: a multiple of 4
         long long i = (long long)blockIdx.x * 256 + threadIdx.x;
@@ -140,10 +146,10 @@ static int copy_blocks(const Geom& g) {
     return (int)(want < 148 * 8 ? want : 148 * 8);
 }
 static void field_in(const float* d, float* p, const Geom& g, cudaStream_t st) {
-    k_field_copy<<<copy_blocks(g), 256, 0, st>>>(d, g.N, p, g.P, g.N, (long long)g.N * g.N);
+    launch_dependent(k_field_copy, copy_blocks(g), 256, 0, st, d, g.N, p, g.P, g.N, (long long)g.N * g.N);
 }
 static void field_out(const float* p, float* d, const Geom& g, cudaStream_t st) {
-    k_field_copy<<<copy_blocks(g), 256, 0, st>>>(p, g.P, d, g.N, g.N, (long long)g.N * g.N);
+    launch_dependent(k_field_copy, copy_blocks(g), 256, 0, st, p, g.P, d, g.N, g.N, (long long)g.N * g.N);
 }
 __global__ void k_fill(float* p, long long n, float v) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -591,7 +597,7 @@ gell_status gell_cells_import(gell_ctx* c, const gell_cell* cells, int n, int on
         src = c->staging;
     }
     if (n > 0) {
-        GELL_KERNEL(c, "k_import", k_import<<<blocks_for(n, kRecBlock), kRecBlock, 0, c->stream>>>(src, c->cur(), n, c->g));
+        GELL_KERNEL(c, "k_import", launch_dependent(k_import, blocks_for(n, kRecBlock), kRecBlock, 0, c->stream, src, c->cur(), n, c->g));
     }
     c->n = n;
     c->sorted_valid = false;
@@ -607,7 +613,7 @@ gell_status gell_cells_export(gell_ctx* c, gell_cell* cells, int capacity, int* 
     int n = c->n;
     if (n > 0) {
         gell_cell* dst = on_device ? cells : c->staging;
-        GELL_KERNEL(c, "k_export", k_export<<<blocks_for(n, kRecBlock), kRecBlock, 0, c->stream>>>(c->cur(), dst, n));
+        GELL_KERNEL(c, "k_export", launch_dependent(k_export, blocks_for(n, kRecBlock), kRecBlock, 0, c->stream, c->cur(), dst, n));
         if (!on_device) {
             GELL_CUDA(c, cudaMemcpyAsync(cells, c->staging, (size_t)n * sizeof(gell_cell),
                                          cudaMemcpyDeviceToHost, c->stream));
@@ -626,7 +632,7 @@ gell_status gell_cells_import_async(gell_ctx* c, const gell_cell* cells, int n) 
     if (n > 0) {
         GELL_CUDA(c, cudaMemcpyAsync(c->staging, cells, (size_t)n * sizeof(gell_cell), cudaMemcpyHostToDevice,
                                      c->xfer));
-        k_import<<<blocks_for(n, kRecBlock), kRecBlock, 0, c->xfer>>>(c->staging, c->cur(), n, c->g);
+        launch_dependent(k_import, blocks_for(n, kRecBlock), kRecBlock, 0, c->xfer, c->staging, c->cur(), n, c->g);
         c->launches++;
         GELL_LAUNCH(c, "k_import");
     }
@@ -645,7 +651,7 @@ gell_status gell_cells_export_async(gell_ctx* c, gell_cell* cells, int capacity,
     const int n = c->n;
     GELL_CUDA(c, cudaStreamWaitEvent(c->xfer, c->cells_ev, 0));
     if (n > 0) {
-        k_export<<<blocks_for(n, kRecBlock), kRecBlock, 0, c->xfer>>>(c->cur(), c->staging, n);
+        launch_dependent(k_export, blocks_for(n, kRecBlock), kRecBlock, 0, c->xfer, c->cur(), c->staging, n);
         c->launches++;
         GELL_LAUNCH(c, "k_export");
         GELL_CUDA(c, cudaMemcpyAsync(cells, c->staging, (size_t)n * sizeof(gell_cell), cudaMemcpyDeviceToHost,

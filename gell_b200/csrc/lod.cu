@@ -1566,9 +1566,17 @@ struct PreArgs {
     float dead;
 };
 
-__global__ void k_rate_reset(PreArgs a) { rate_reset_body(a, blockIdx.x, gridDim.x); }
+__global__ void k_rate_reset(PreArgs a) {
+    grid_dep_wait();
+    grid_dep_launch();
+    rate_reset_body(a, blockIdx.x, gridDim.x);
+}
 
-__global__ void k_rate_accum(CellsSoA c, int n, PreArgs a) { rate_accum_body(c, n, a, blockIdx.x); }
+__global__ void k_rate_accum(CellsSoA c, int n, PreArgs a) {
+    grid_dep_wait();
+    grid_dep_launch();
+    rate_accum_body(c, n, a, blockIdx.x);
+}
 
 int g_num_sms = 0;
 int num_sms() {
@@ -1616,10 +1624,10 @@ gell_status prelod(gell_ctx* c, int sub) {
     }
     a.g = c->g;
     a.dead = c->P.dead_uptake_factor;
-    GELL_KERNEL(c, "k_rate_reset", k_rate_reset<<<num_sms() * 4, 256, 0, c->stream>>>(a));
+    GELL_KERNEL(c, "k_rate_reset", launch_dependent(k_rate_reset, num_sms() * 4, 256, 0, c->stream, a));
     for (int s = 0; s < a.nsub; ++s) GELL_CUDA(c, cudaMemsetAsync(a.count[s], 0, 4, c->stream));
     if (c->n > 0) {
-        GELL_KERNEL(c, "k_rate_accum", k_rate_accum<<<blocks_for(c->n, 256), 256, 0, c->stream>>>(c->cur(), c->n, a));
+        GELL_KERNEL(c, "k_rate_accum", launch_dependent(k_rate_accum, blocks_for(c->n, 256), 256, 0, c->stream, c->cur(), c->n, a));
     }
     c->rate_valid = true;
     return GELL_OK;

@@ -18,19 +18,35 @@ namespace gell {
 namespace {
 
 __global__ void k_keys(CellsSoA c, int n, Geom g, uint32_t* __restrict__ keys, int* __restrict__ epoch) {
+    grid_dep_wait();
+    grid_dep_launch();
     keys_body(c, n, g, keys, epoch, blockIdx.x);
 }
 
-__global__ void __launch_bounds__(kOneThreads, 1) k_sort_one(const __grid_constant__ OneJob a) { sort_one_body(a); }
+__global__ void __launch_bounds__(kOneThreads, 1) k_sort_one(const __grid_constant__ OneJob a) {
+    grid_dep_wait();
+    grid_dep_launch();
+    sort_one_body(a);
+}
 
 __global__ void k_gather(CellsSoA s, CellsSoA d, const uint32_t* __restrict__ keys,
                          const uint32_t* __restrict__ perm, int n, int4* __restrict__ bins,
                          const int* __restrict__ epoch_p) {
+    grid_dep_wait();
+    grid_dep_launch();
     gather_body(s, d, keys, perm, n, bins, epoch_p, blockIdx.x);
 }
 
-__global__ void __launch_bounds__(kForceThreads) k_force_move(MechArgs a) { force_move_body(a, blockIdx.x); }
-__global__ void __launch_bounds__(kForceThreads) k_force_warp(MechArgs a) { force_move_warp_body(a, blockIdx.x); }
+__global__ void __launch_bounds__(kForceThreads) k_force_move(MechArgs a) {
+    grid_dep_wait();
+    grid_dep_launch();
+    force_move_body(a, blockIdx.x);
+}
+__global__ void __launch_bounds__(kForceThreads) k_force_warp(MechArgs a) {
+    grid_dep_wait();
+    grid_dep_launch();
+    force_move_warp_body(a, blockIdx.x);
+}
 
 // A warp per cell up to here, a thread per cell beyond (us, both measured: 2,000 cells 9 against 32, 10,000 14
 // against 34, 30,000 25 against 36, 60,000 41 against 35).
@@ -77,16 +93,16 @@ gell_status fm_update(gell_ctx* c) {
     if (n > 0) {
         if (n <= kOneCells) {
             GELL_CUDA(c, cudaFuncSetAttribute(k_sort_one, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneSmem));
-            GELL_KERNEL(c, "k_sort_one", k_sort_one<<<1, kOneThreads, kOneSmem, c->stream>>>(one_job(c)));
+            GELL_KERNEL(c, "k_sort_one", launch_dependent(k_sort_one, 1, kOneThreads, kOneSmem, c->stream, one_job(c)));
             c->sort.which = 0;
         } else {
-            GELL_KERNEL(c, "k_keys", k_keys<<<blocks_for(n, 256), 256, 0, c->stream>>>(c->cur(), n, c->g, c->sort.keys[0],
+            GELL_KERNEL(c, "k_keys", launch_dependent(k_keys, blocks_for(n, 256), 256, 0, c->stream, c->cur(), n, c->g, c->sort.keys[0],
                                                                                     c->dev_epoch));
             gell_status st = radix_sort(c, n, key_bits(c->g.N), true);
             if (st != GELL_OK) return st;
         }
         const int w = c->sort.which;
-        GELL_KERNEL(c, "k_gather", k_gather<<<blocks_for(n, 256), 256, 0, c->stream>>>(c->cur(), c->alt(), c->sort.keys[w], c->sort.vals[w], n,
+        GELL_KERNEL(c, "k_gather", launch_dependent(k_gather, blocks_for(n, 256), 256, 0, c->stream, c->cur(), c->alt(), c->sort.keys[w], c->sort.vals[w], n,
                                                               c->bins, c->dev_epoch));
         c->swap_all();
         MechArgs a;
@@ -105,7 +121,7 @@ gell_status fm_update(gell_ctx* c) {
         a.sure = a.ra_ratio > 0.0 ? 1.f - 0x1p-18f : -1.f;
         a.half_dt = c->P.mechanics_dt / 2.f;
         const int per = force_block(n);
-        GELL_KERNEL(c, "k_force_move", (per < kForceThreads ? k_force_warp : k_force_move)<<<blocks_for(n, per), kForceThreads, 0, c->stream>>>(a));
+        GELL_KERNEL(c, "k_force_move", launch_dependent((per < kForceThreads ? k_force_warp : k_force_move), blocks_for(n, per), kForceThreads, 0, c->stream, a));
         c->sign.swap();
         c->mesh.swap();
         c->posr.swap();
@@ -162,6 +178,8 @@ struct KeysBatch {
     KeysJob job[kBatchMembers];
 };
 __global__ void k_keys_batch(const __grid_constant__ KeysBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     int local;
     const KeysJob& j = b.job[member_of(b.map, blockIdx.x, local)];
     keys_body(j.c, j.n, j.g, j.keys, j.epoch, local);
@@ -180,16 +198,22 @@ struct SortBatch {
     SortJob job[kBatchMembers];
 };
 __global__ void __launch_bounds__(kSortThreads) k_hist_batch(const __grid_constant__ SortBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     int local;
     const SortJob& j = b.job[member_of(b.tiles, blockIdx.x, local)];
     hist_body(j.kin, j.n, j.shift, j.R, j.hist, j.nb, local);
 }
 __global__ void __launch_bounds__(kSortThreads) k_digit_scan_batch(const __grid_constant__ SortBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     int local;
     const SortJob& j = b.job[member_of(b.digits, blockIdx.x, local)];
     digit_scan_body(j.hist, j.nb, j.hist + (size_t)j.R * j.nb, local);
 }
 __global__ void __launch_bounds__(kSortThreads) k_scatter_batch(const __grid_constant__ SortBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     int local;
     const SortJob& j = b.job[member_of(b.tiles, blockIdx.x, local)];
     scatter_body(j.kin, j.vin, j.kout, j.vout, j.n, j.shift, j.R, j.hist, j.nb, j.hist + (size_t)j.R * j.nb, j.iota,
@@ -200,6 +224,8 @@ struct OneBatch {
     OneJob job[kBatchMembers];
 };
 __global__ void __launch_bounds__(kOneThreads, 1) k_sort_one_batch(const __grid_constant__ OneBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     sort_one_body(b.job[blockIdx.x]);
 }
 
@@ -216,6 +242,8 @@ struct GatherBatch {
     GatherJob job[kBatchMembers];
 };
 __global__ void k_gather_batch(const __grid_constant__ GatherBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     int local;
     const GatherJob& j = b.job[member_of(b.map, blockIdx.x, local)];
     gather_body(j.s, j.d, j.keys, j.perm, j.n, j.bins, j.epoch, local);
@@ -226,11 +254,15 @@ struct ForceBatch {
     MechArgs job[kBatchMembers];
 };
 __global__ void __launch_bounds__(kForceThreads) k_force_move_batch(const __grid_constant__ ForceBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     int local;
     const MechArgs& j = b.job[member_of(b.map, blockIdx.x, local)];
     force_move_body(j, local);
 }
 __global__ void __launch_bounds__(kForceThreads) k_force_warp_batch(const __grid_constant__ ForceBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     int local;
     const MechArgs& j = b.job[member_of(b.map, blockIdx.x, local)];
     force_move_warp_body(j, local);
@@ -258,10 +290,14 @@ __global__ void k_rate_reset_batch(const __grid_constant__ PreBatch b) {
     rate_reset_body(b.job[blockIdx.y], blockIdx.x, gridDim.x);
 }
 __global__ void k_zero_counts_batch(const __grid_constant__ PreBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     const int m = threadIdx.x / kBatchSub, s = threadIdx.x % kBatchSub;
     if (m < b.map.nm && s < b.job[m].nsub) *b.job[m].count[s] = 0;
 }
 __global__ void k_rate_accum_batch(const __grid_constant__ PreBatch b) {
+    grid_dep_wait();
+    grid_dep_launch();
     int local;
     const PreJob& j = b.job[member_of(b.map, blockIdx.x, local)];
     rate_accum_body(j.c, j.n, j, local);
@@ -313,7 +349,7 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
         }
         if (small > 0) {
             GELL_CUDA(c0, cudaFuncSetAttribute(k_sort_one_batch, cudaFuncAttributeMaxDynamicSharedMemorySize, kOneSmem));
-            GELL_KERNEL(c0, "k_sort_one_batch", k_sort_one_batch<<<small, kOneThreads, kOneSmem, st>>>(ob));
+            GELL_KERNEL(c0, "k_sort_one_batch", launch_dependent(k_sort_one_batch, small, kOneThreads, kOneSmem, st, ob));
         }
         if (!large.empty()) {
             KeysBatch kb{};
@@ -324,7 +360,7 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
                 kb.job[k] = KeysJob{c->cur(), c->sort.keys[0], c->dev_epoch, c->g, c->n};
             }
             const int kblocks = fill_map(kb.map, kb_blocks);
-            GELL_KERNEL(c0, "k_keys_batch", k_keys_batch<<<kblocks, 256, 0, st>>>(kb));
+            GELL_KERNEL(c0, "k_keys_batch", launch_dependent(k_keys_batch, kblocks, 256, 0, st, kb));
         }
 
         // the sort of the others: each member's own digit width and pass count (radix_sort's rule)
@@ -353,10 +389,10 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
             }
             const int ntiles = fill_map(sb.tiles, tiles);
             const int ndigits = fill_map(sb.digits, digits);
-            GELL_KERNEL(c0, "k_hist_batch", k_hist_batch<<<ntiles, kSortThreads, 0, st>>>(sb));
+            GELL_KERNEL(c0, "k_hist_batch", launch_dependent(k_hist_batch, ntiles, kSortThreads, 0, st, sb));
             if (ndigits > 0)
-                GELL_KERNEL(c0, "k_digit_scan_batch", k_digit_scan_batch<<<ndigits, kSortThreads, 0, st>>>(sb));
-            GELL_KERNEL(c0, "k_scatter_batch", k_scatter_batch<<<ntiles, kSortThreads, 0, st>>>(sb));
+                GELL_KERNEL(c0, "k_digit_scan_batch", launch_dependent(k_digit_scan_batch, ndigits, kSortThreads, 0, st, sb));
+            GELL_KERNEL(c0, "k_scatter_batch", launch_dependent(k_scatter_batch, ntiles, kSortThreads, 0, st, sb));
             for (int i : who) {
                 in[i] ^= 1;
                 iota[i] = 0;
@@ -372,7 +408,7 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
                                   c->n};
             c->swap_all();
         }
-        GELL_KERNEL(c0, "k_gather_batch", k_gather_batch<<<gblocks, 256, 0, st>>>(gb));
+        GELL_KERNEL(c0, "k_gather_batch", launch_dependent(k_gather_batch, gblocks, 256, 0, st, gb));
 
         long long cells = 0;
         for (gell_ctx* c : fm) cells += c->n;
@@ -404,7 +440,7 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
             c->oldf.swap();
         }
         GELL_KERNEL(c0, "k_force_move_batch",
-                    (per < kForceThreads ? k_force_warp_batch : k_force_move_batch)<<<fblocks, kForceThreads, 0, st>>>(fb));
+                    launch_dependent((per < kForceThreads ? k_force_warp_batch : k_force_move_batch), fblocks, kForceThreads, 0, st, fb));
     }
     for (gell_ctx* c : ms) {
         c->sorted_valid = true;
@@ -441,8 +477,8 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
         const int ablocks = fill_map(pb.map, blocks);
         GELL_KERNEL(c0, "k_rate_reset_batch",
                     k_rate_reset_batch<<<dim3(kResetBlocks, (unsigned)pm.size()), 256, 0, st>>>(pb));
-        GELL_KERNEL(c0, "k_zero_counts_batch", k_zero_counts_batch<<<1, 256, 0, st>>>(pb));
-        if (ablocks > 0) GELL_KERNEL(c0, "k_rate_accum_batch", k_rate_accum_batch<<<ablocks, 256, 0, st>>>(pb));
+        GELL_KERNEL(c0, "k_zero_counts_batch", launch_dependent(k_zero_counts_batch, 1, 256, 0, st, pb));
+        if (ablocks > 0) GELL_KERNEL(c0, "k_rate_accum_batch", launch_dependent(k_rate_accum_batch, ablocks, 256, 0, st, pb));
         for (gell_ctx* c : pm) c->rate_valid = true;
     }
     return GELL_OK;

@@ -19,11 +19,15 @@ namespace gell {
 namespace {
 __global__ void __launch_bounds__(kSortThreads) k_hist(const uint32_t* __restrict__ keys, int n, int shift,
                                                    int R, uint32_t* __restrict__ hist, int nb) {
+    grid_dep_wait();
+    grid_dep_launch();
     hist_body(keys, n, shift, R, hist, nb, blockIdx.x);
 }
 
 __global__ void __launch_bounds__(kSortThreads) k_digit_scan(uint32_t* __restrict__ hist, int nb,
                                                          uint32_t* __restrict__ totals) {
+    grid_dep_wait();
+    grid_dep_launch();
     digit_scan_body(hist, nb, totals, blockIdx.x);
 }
 
@@ -31,6 +35,8 @@ __global__ void __launch_bounds__(kSortThreads) k_scatter(const uint32_t* __rest
                                                       uint32_t* __restrict__ kout, uint32_t* __restrict__ vout, int n,
                                                       int shift, int R, const uint32_t* __restrict__ offs, int nb,
                                                       const uint32_t* __restrict__ totals, int iota) {
+    grid_dep_wait();
+    grid_dep_launch();
     scatter_body(kin, vin, kout, vout, n, shift, R, offs, nb, totals, iota, blockIdx.x);
 }
 
@@ -53,11 +59,11 @@ gell_status radix_sort(gell_ctx* c, int n, int bits, bool vals_are_iota) {
     bool iota = vals_are_iota;
     for (int p = 0; p < passes; ++p) {
         const int shift = p * d;
-        GELL_KERNEL(c, "k_hist", k_hist<<<nb, kSortThreads, 0, c->stream>>>(S.keys[in], n, shift, R, S.hist, nb));
+        GELL_KERNEL(c, "k_hist", launch_dependent(k_hist, nb, kSortThreads, 0, c->stream, S.keys[in], n, shift, R, S.hist, nb));
         uint32_t* totals = S.hist + (size_t)R * nb;
         if (nb > kSortScanTiles)
-            GELL_KERNEL(c, "k_digit_scan", k_digit_scan<<<R, kSortThreads, 0, c->stream>>>(S.hist, nb, totals));
-        GELL_KERNEL(c, "k_scatter", k_scatter<<<nb, kSortThreads, 0, c->stream>>>(S.keys[in], S.vals[in], S.keys[in ^ 1], S.vals[in ^ 1], n, shift,
+            GELL_KERNEL(c, "k_digit_scan", launch_dependent(k_digit_scan, R, kSortThreads, 0, c->stream, S.hist, nb, totals));
+        GELL_KERNEL(c, "k_scatter", launch_dependent(k_scatter, nb, kSortThreads, 0, c->stream, S.keys[in], S.vals[in], S.keys[in ^ 1], S.vals[in ^ 1], n, shift,
                                                    R, S.hist, nb, totals, iota ? 1 : 0));
         iota = false;
         in ^= 1;
