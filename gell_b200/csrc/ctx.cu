@@ -3,6 +3,8 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
+#include <vector>
 #include <cudaTypedefs.h>
 #include <new>
 
@@ -242,6 +244,64 @@ void gell_substrate_oxygen(gell_substrate* s) {
     s->init = 38.f;
 }
 
+// Pinned words, one per context, into which birth and death write their counts.  A copy to pageable memory
+// costs 12 us a call, and pinning a word of its own 1.7 ms a context: words come from pages of 64 that all
+// contexts share; the first page stays until the process ends, others go when their last word comes back.
+// A page that the runtime no longer knows (the device was reset) is dropped.
+class CountWords {
+public:
+    int* take() {
+        std::lock_guard<std::mutex> lock(m_);
+        for (size_t k = 0; k < pages_.size();) {
+            cudaPointerAttributes at{};
+            if (cudaPointerGetAttributes(&at, pages_[k].base) != cudaSuccess || at.type != cudaMemoryTypeHost) {
+                cudaGetLastError();
+                pages_.erase(pages_.begin() + (long)k);
+                continue;
+            }
+            if (~pages_[k].used) return word(pages_[k]);
+            ++k;
+        }
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, 64 * kStride * sizeof(int), cudaHostAllocPortable) != cudaSuccess) return nullptr;
+        pages_.push_back(Page{static_cast<int*>(p), 0});
+        return word(pages_.back());
+    }
+    void give(int* w) {
+        if (!w) return;
+        std::lock_guard<std::mutex> lock(m_);
+        for (size_t k = 0; k < pages_.size(); ++k) {
+            Page& p = pages_[k];
+            if (w < p.base || w >= p.base + 64 * kStride) continue;
+            p.used &= ~(1ull << ((w - p.base) / kStride));
+            if (!p.used && pages_.size() > 1) {
+                cudaFreeHost(p.base);
+                pages_.erase(pages_.begin() + (long)k);
+            }
+            return;
+        }
+    }
+
+private:
+    static constexpr int kStride = 16;  // 64 bytes a word
+    struct Page {
+        int* base;
+        unsigned long long used;
+    };
+    static int* word(Page& p) {
+        int k = 0;
+        while (p.used >> k & 1) ++k;
+        p.used |= 1ull << k;
+        return p.base + k * kStride;
+    }
+    std::mutex m_;
+    std::vector<Page> pages_;
+};
+static CountWords& count_words() {
+    static CountWords* words = new CountWords;  // never destroyed: contexts may be freed while the process ends
+    return *words;
+}
+
 static void free_all(gell_ctx* c) {
     auto f = [](void* p) { if (p) cudaFree(p); };
     for (int b = 0; b < 2; ++b) {
@@ -258,7 +318,7 @@ static void free_all(gell_ctx* c) {
     surrogate_free(c);
     for (auto& s : c->subs) { f(s.p); f(s.rate); f(s.EF); f(s.FRS); f(s.line_flag); f(s.line_list); f(s.line_count); }
     f(c->xorwow); f(c->flags); f(c->counts); f(c->dev_err);
-    if (c->total) cudaFreeHost(c->total);
+    count_words().give(c->total);
     f(c->staging);
     for (auto& p : c->prof) { cudaEventDestroy(p.a); cudaEventDestroy(p.b); }
     for (auto e : c->ev_pool) cudaEventDestroy(e);
@@ -342,7 +402,7 @@ gell_status gell_create(const gell_params* params, gell_ctx** out) {
     A((void**)&c->dev_err, 64);
     A((void**)&c->staging, cap * sizeof(gell_cell));
     if (P.rng_mode == GELL_RNG_XORWOW) A((void**)&c->xorwow, cap * sizeof(curandState));
-    if (st == GELL_OK && cudaHostAlloc((void**)&c->total, 64, cudaHostAllocDefault) != cudaSuccess) st = GELL_ERR_CUDA;
+    if (st == GELL_OK && !(c->total = count_words().take())) st = GELL_ERR_CUDA;
     if (st != GELL_OK) {
         free_all(c);
         delete c;

@@ -10,7 +10,8 @@
 // The numbers come without a scan of their own: the first kernel leaves a count per block, and a
 // block of the second adds the counts before it (at most 4 per thread at 1M cells, from L2) and
 // ranks its own 1,024 cells by votes.  Two launches each for birth and death, where flags, two-level
-// scan and use were five (50,000 cells, import and export with them: 112 -> 68 us; 1M: 200 -> 150); the total goes to a pinned host word.
+// scan and use were five (50,000 cells, import and export with them: 112 -> 68 us; 1M: 200 -> 150).
+// The total goes to a pinned word.
 //
 // Draws: GELL_RNG_XORWOW keeps one curand XORWOW state per slot initialised with
 // curand_init(seed, slot, 0) and draws exactly as the reference does (u, then two draws for the

@@ -39,3 +39,24 @@ def test_birth_slots_at_block_edges(n, cap):
     for f in ("sign", "phase", "V", "Vf", "Vcs", "Vns", "cell_clock"):
         np.testing.assert_array_equal(out[f], oc[f][:on])
     np.testing.assert_allclose(out["pos"], oc["pos"][:on], rtol=1e-6, atol=1e-4)  # CUDA's sinf, acosf and pow
+
+
+def test_counts_of_many_contexts_side_by_side():
+    """The counts come back through words shared by all contexts, 64 to a page: more contexts than a page has
+    words, destroyed and created again in between, each with its own number of live cells."""
+    def make(k):
+        cells = eventful_cells(8, 10.0, 300 + k, k)
+        cells["sign"] = 0
+        cells["sign"][:2 + k] = 1
+        sim = gb.Simulation(voxel_num=8, voxel_length=10.0, max_cell_num=512)
+        sim.import_cells(cells)
+        return sim
+
+    sims = {k: make(k) for k in range(70)}
+    for k in range(0, 70, 3):
+        sims.pop(k).close()
+    for k in range(0, 70, 6):
+        sims[k] = make(k)
+    for k in sorted(sims, reverse=True):
+        assert sims[k].CellDeath_kernel() == 2 + k
+        sims.pop(k).close()
