@@ -149,7 +149,7 @@ __device__ __forceinline__ void live_move(const MechArgs& a, int i, const float4
 // for a sixth of its lanes.  The walk therefore only decides which candidates are accepted, from |dp|^2 and
 // bounds of the cutoff's square that leave the distance itself to a margin of 2^-18, and lists those that act;
 // the lists are worked through afterwards, entry by entry.  What bounds it is the issue of instructions (5,770 a
-// warp before, 4,800 now, 70% of the cycles); 1M cells 237 -> 207 us, 100,000 57 -> 43.
+// warp before, 4,660 now, 67% of the cycles); 1M cells 237 -> 207 us, 100,000 57 -> 43.
 constexpr int kForceThreads = 256;
 constexpr int kForceList = 16;  // entries; a full list is worked off before the walk goes on
 // above hi, d >= t is certain; up to lo, d < t is: margins far above the roundings between |dp|^2 + 0.0001 and d
