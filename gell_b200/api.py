@@ -141,6 +141,7 @@ def load_library() -> ctypes.CDLL:
     L.gell_cell_death.argtypes = [P, P]
     L.gell_mechanics_step.argtypes = [P, ctypes.c_int]
     L.gell_sync.argtypes = [P]
+    L.gell_debug_conv_units.argtypes = [P, ctypes.c_int, ctypes.c_int]
     L.gell_debug_dump.argtypes = [P, ctypes.c_int, ctypes.c_int, P, ctypes.c_size_t]
     L.gell_status_string.argtypes = [ctypes.c_int]
     L.gell_status_string.restype = ctypes.c_char_p
@@ -168,7 +169,7 @@ def load_library() -> ctypes.CDLL:
                  "gell_cells_import", "gell_cells_export", "gell_cell_count", "gell_field_import",
                  "gell_field_export", "gell_fm_update", "gell_prelod", "gell_lod_solver",
                  "gell_cell_birth", "gell_cell_death", "gell_mechanics_step", "gell_sync",
-                 "gell_debug_dump", "gell_profile_enable", "gell_profile_read", "gell_launch_count",
+                 "gell_debug_dump", "gell_debug_conv_units", "gell_profile_enable", "gell_profile_read", "gell_launch_count",
                  "gell_selftest_division", "gell_set_option", "gell_selftest_timeout", "gell_cells_import_async",
                  "gell_cells_export_async", "gell_wait_transfers", "gell_run_mechanics",
                  "gell_write_cells_csv", "gell_save_cells_csv", "gell_save_field_csv",
@@ -485,6 +486,10 @@ class Simulation:
         return out
 
     # -- parity support
+    def debug_conv_units(self, lines: int = 0, ctas: int = 0) -> None:
+        """Units of `lines` output lines and at most `ctas` CTAs for the surrogate's convolutions (0: their choice)."""
+        self._check(self.lib.gell_debug_conv_units(self.h, lines, ctas), "gell_debug_conv_units")
+
     def _dump(self, what: int, arg: int, dtype, count: int) -> np.ndarray:
         out = np.zeros(max(count, 1), dtype)
         self._check(self.lib.gell_debug_dump(self.h, what, arg, P(out.ctypes.data), out.nbytes),

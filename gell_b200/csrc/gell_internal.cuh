@@ -114,6 +114,7 @@ struct gell_ctx {
 
     std::vector<gell::Substrate> subs;
     gell::SurrogateState* sur[8] = {};  // per substrate, created by gell_surrogate_load
+    int conv_unit_lines = 0, conv_ctas = 0;  // gell_debug_conv_units (0: the launch's own choice)
     int sur_input = 0;                  // GELL_OPT_SURROGATE_INPUT for surrogates loaded from now on
     bool rate_valid = false;
     bool exact_chain = false;  // GELL_OPT_EXACT_CHAIN

@@ -348,6 +348,12 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv3(const __grid_constant
             nz = w.z1 - w.z0;
         }
         while (ok && u < U) {
+            // a unit of one line leaves its accumulator's hand-over pending, and the next unit's first line
+            // would wait for that accumulator
+            if (m == cacc) {
+                commit();
+                csl = cacc = -1;
+            }
             ok = mbar_wait(&full[sl], gph, a.err, 23);
             if (ok) ok = wait_acc(m, nz);
             if (!ok) break;
@@ -1040,6 +1046,7 @@ static void pack_layer(const float* W, const LayerShape& s, std::vector<uint16_t
 
 // Lines per unit: as many as possible (a unit loads two row groups more than it has lines), but few enough
 // that the units fill the last round of CTAs; the cost of a round is its lines plus those two groups.
+// The last unit along z can be of any length from one line on.
 static int unit_lines(int N, int sms) {
     int best = kUnitZ;
     long long cost = -1;
@@ -1051,6 +1058,22 @@ static int unit_lines(int N, int sms) {
         }
     }
     return best;
+}
+
+// Lines per unit and CTAs of a k_conv3 or k_wgrad launch (or what gell_debug_conv_units asks for).
+struct UnitPlan {
+    int tiles_x, unit_z, grid;
+};
+static gell_status unit_plan(gell_ctx* c, UnitPlan* p) {
+    const int N = c->g.N;
+    int sms = 0;
+    GELL_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
+    p->tiles_x = (N + kTileM - 1) / kTileM;
+    p->unit_z = c->conv_unit_lines > 0 ? c->conv_unit_lines : unit_lines(N, sms);
+    const long long units = (long long)p->tiles_x * ((N + p->unit_z - 1) / p->unit_z) * N;
+    const int most = c->conv_ctas > 0 && c->conv_ctas < sms ? c->conv_ctas : sms;
+    p->grid = (int)(units < most ? units : most);
+    return GELL_OK;
 }
 
 template <int CIN8, int NOUT, int MODE>
@@ -1073,16 +1096,14 @@ static gell_status launch_conv(gell_ctx* c, const char* name, const PlaneMaps& i
     a.P = c->g.P;
     a.PN = c->g.PN;
     a.nvox = c->nvox;
-    a.tiles_x = (c->g.N + kTileM - 1) / kTileM;
     a.scale = scale;
     a.bval = bval;
     a.err = c->dev_err;
-    int sms = 0;
-    GELL_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-    a.unit_z = unit_lines(c->g.N, sms);
-    const long long units = (long long)a.tiles_x * ((c->g.N + a.unit_z - 1) / a.unit_z) * c->g.N;
-    const int grid = (int)(units < sms ? units : sms);
-    GELL_KERNEL(c, name, (k_conv3<CIN8, NOUT, MODE><<<grid, kConvThreads, L::kBytes, c->stream>>>(a)));
+    UnitPlan plan{};
+    if (gell_status st = unit_plan(c, &plan)) return st;
+    a.tiles_x = plan.tiles_x;
+    a.unit_z = plan.unit_z;
+    GELL_KERNEL(c, name, (k_conv3<CIN8, NOUT, MODE><<<plan.grid, kConvThreads, L::kBytes, c->stream>>>(a)));
     return GELL_OK;
 }
 
@@ -1165,20 +1186,17 @@ template <int BP>
 static gell_status launch_wgrad(gell_ctx* c, TrainState* T, const LayerShape& sh, const PlaneMaps& A, const PlaneMaps& B,
                                 bool gradient_a, float* out) {
     using L = WgradSmem<BP>;
-    const int N = c->g.N;
     WgradArgs a{};
     a.a = A.all;
     a.b = B.all;
     a.partial = T->partial;
-    a.N = N;
-    a.tiles_x = (N + kTileM - 1) / kTileM;
+    a.N = c->g.N;
     a.err = c->dev_err;
-    int sms = 0;
-    GELL_CUDA(c, cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device));
-    a.unit_z = unit_lines(N, sms);
-    const long long units = (long long)a.tiles_x * ((N + a.unit_z - 1) / a.unit_z) * N;
-    int grid = (int)(units < sms ? units : sms);
-    if (grid > kWgCtas) grid = kWgCtas;
+    UnitPlan plan{};
+    if (gell_status st = unit_plan(c, &plan)) return st;
+    a.tiles_x = plan.tiles_x;
+    a.unit_z = plan.unit_z;
+    const int grid = plan.grid < kWgCtas ? plan.grid : kWgCtas;
     GELL_CUDA(c, cudaFuncSetAttribute(k_wgrad<BP>, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kBytes));
     GELL_KERNEL(c, BP == 2 ? "k_wgrad_thin" : "k_wgrad", (k_wgrad<BP><<<grid, kWgThreads, L::kBytes, c->stream>>>(a)));
     const int n = 27 * 256 * BP;
@@ -1475,6 +1493,14 @@ gell_status gell_surrogate_run_layers(gell_ctx* c, int sub, int layers) {
     SurrogateState* S = c->sur[sub];
     if (!S) return fail(c, GELL_ERR_INVALID_ARG, "no surrogate loaded for this substrate");
     return run_layers(c, sub, S, layers);
+}
+
+gell_status gell_debug_conv_units(gell_ctx* c, int lines, int ctas) {
+    if (!c) return GELL_ERR_INVALID_ARG;
+    if (lines < 0 || lines > kUnitZ || ctas < 0) return fail(c, GELL_ERR_INVALID_ARG, "convolution units outside 0..16 lines");
+    c->conv_unit_lines = lines;
+    c->conv_ctas = ctas;
+    return GELL_OK;
 }
 
 gell_status gell_surrogate_read(gell_ctx* c, int sub, int which, void* host, long long bytes) {

@@ -227,6 +227,10 @@ enum {
     GELL_DUMP_EF = 5
 };
 gell_status gell_debug_dump(gell_ctx* ctx, int what, int arg, void* out, size_t bytes);
+/* Test support: the surrogate's convolutions and weight gradients take units of `lines` (1..16) output
+ * lines along z and at most `ctas` CTAs, so that a small grid reaches any sequence of units that a large
+ * one gives a CTA; 0 leaves either to the launch.  Results do not change (gradients: other sum order). */
+gell_status gell_debug_conv_units(gell_ctx* ctx, int lines, int ctas);
 
 /* Per-kernel timing.  When enabled, every kernel this library launches is bracketed by CUDA events
  * on the context's stream; gell_profile_read synchronises and reports, per kernel name, the number
