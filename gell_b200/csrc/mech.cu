@@ -37,7 +37,7 @@ __global__ void k_gather(CellsSoA s, CellsSoA d, const uint32_t* __restrict__ ke
     gather_body(s, d, keys, perm, n, bins, epoch_p, blockIdx.x);
 }
 
-__global__ void __launch_bounds__(kForceThreads) k_force_move(MechArgs a) {
+__global__ void __launch_bounds__(kForceThreads, 5) k_force_move(MechArgs a) {
     grid_dep_wait();
     grid_dep_launch();
     force_move_body(a, blockIdx.x);
@@ -253,7 +253,7 @@ struct ForceBatch {
     BlockMap map;
     MechArgs job[kBatchMembers];
 };
-__global__ void __launch_bounds__(kForceThreads) k_force_move_batch(const __grid_constant__ ForceBatch b) {
+__global__ void __launch_bounds__(kForceThreads, 5) k_force_move_batch(const __grid_constant__ ForceBatch b) {
     grid_dep_wait();
     grid_dep_launch();
     int local;

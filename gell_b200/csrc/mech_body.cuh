@@ -1,9 +1,11 @@
 // mech_body.cuh — the per-block bodies of the mechanics kernels (mech.cu: keys, gather, force and
 // move; sort.cu: the radix sort's histogram, digit scan and scatter; lod.cu: the uptake map), shared
-// by the one-context kernels and the ensemble's batched kernels (mech_batch.cu), which run the same
+// by the one-context kernels and the ensemble's batched kernels (mech.cu), which run the same
 // body for block `blk` of one member.  Each body is the kernel it came from with blockIdx.x
 // replaced by `blk`, so a batched launch computes what the member's own launches compute.
 #pragma once
+
+#include <type_traits>
 
 #include "async_copy.cuh"
 #include "gell_internal.cuh"
@@ -148,10 +150,19 @@ __device__ __forceinline__ void live_move(const MechArgs& a, int i, const float4
 // lane's and ~9 accepted ones, so that with the force computed in the walk the warp issued the force's code
 // for a sixth of its lanes.  The walk therefore only decides which candidates are accepted, from |dp|^2 and
 // bounds of the cutoff's square that leave the distance itself to a margin of 2^-18, and lists those that act;
-// the lists are worked through afterwards, entry by entry.  What bounds it is the issue of instructions (5,770 a
-// warp before, 4,660 now, 67% of the cycles); 1M cells 237 -> 207 us, 100,000 57 -> 43.
+// the lists are worked through afterwards, entry by entry.  What bounds it is the issue of instructions;
+// 1M cells 237 us with the force in the walk, 204 so, 100,000 54 and 41.  Five blocks an SM (48 registers)
+// rather than four (60): 204 against 211 us at 1M cells, 573 against 603 at 3M.
+//
+// Where many candidates are accepted the list is the detour: a warp whose bins promise more than a list holds
+// (kForceCrowd accepted candidates, from the count of a bin near by and the cutoff's sphere) computes the
+// forces in the walk, and a lane whose list fills up leaves the walk, waits until the warp has worked its
+// lists off, and goes on from there in that way.  (Lists worked off by each lane by itself in the middle of
+// its walk took the warp up to 32 lists' time: 1M cells at random, 3, 8 and 37 to a bin, 1,550, 4,300 and
+// 18,400 us; all forces in the walk 580, 1,090 and 3,560; so 568, 1,078 and 3,490.)
 constexpr int kForceThreads = 256;
-constexpr int kForceList = 16;  // entries; a full list is worked off before the walk goes on
+constexpr int kForceList = 24;   // entries
+constexpr int kForceCrowd = 24;  // accepted candidates, estimated
 // above hi, d >= t is certain; up to lo, d < t is: margins far above the roundings between |dp|^2 + 0.0001 and d
 struct Cutoff {
     float t, hi, lo;
@@ -163,8 +174,9 @@ __device__ __forceinline__ Cutoff cutoff_bounds(float t, float sure) {
 __device__ __forceinline__ void force_move_body(const MechArgs& a, int blk) {
     __shared__ int list[kForceList][kForceThreads];
     const int i = blk * blockDim.x + threadIdx.x;
+    const uint8_t sg = i < a.n ? a.cur.sign[i] : 0;
+    const unsigned live = __ballot_sync(FULL, sg != 0);
     if (i >= a.n) return;
-    const uint8_t sg = a.cur.sign[i];
     const float4 pr = a.cur.posr[i];
     const float4 of = a.cur.oldf[i];
     if (!sg) {
@@ -178,52 +190,79 @@ __device__ __forceinline__ void force_move_body(const MechArgs& a, int blk) {
     float fx = 0.f, fy = 0.f, fz = 0.f;
     Cutoff c = cutoff_bounds(a.max_dist, a.max_dist > 0.f ? 1.f - 0x1p-18f : -1.f);
     int cnt = 0;
-    auto work_off = [&] {
-#pragma unroll 1
-        for (int k = 0; k < cnt; ++k) {
-            const float4 q = a.cur.posr[list[k][threadIdx.x]];
-            const Pair v = pair_of(pr, q);
-            const float d = pair_dist(v.ss);
-            const float R = pair_reach(q.w, pr.w);
-            const float own = cutoff_of(a, R);
-            if (d >= own) continue;
-            const float cf = pair_coef(a, d, R, own);
-            fx = __fmaf_rn(v.dx, cf, fx);
-            fy = __fmaf_rn(v.dy, cf, fy);
-            fz = __fmaf_rn(v.dz, cf, fz);
-        }
-        cnt = 0;
+    auto add = [&](const Pair& v, float d, float R, float own) {
+        const float cf = pair_coef(a, d, R, own);
+        fx = __fmaf_rn(v.dx, cf, fx);
+        fy = __fmaf_rn(v.dy, cf, fy);
+        fz = __fmaf_rn(v.dz, cf, fz);
     };
-    // the 27 bins in the reference's order: xi outer, then yi, then zi; the three of a column requested at once
+    // The walk over the 27 bins in the reference's order: xi outer, then yi, then zi; the three of a column
+    // requested at once.  It begins at candidate j0 of bin z0 of column o0, and leaves there where it stood
+    // when the list was full (o0 = 9: at its end).
+    int o0 = 0, z0 = 0, j0 = 0;
+    auto walk = [&](auto listed) {
 #pragma unroll 1
-    for (int o = 0; o < 9; ++o) {
-        const int xi = b.x - 1 + o / 3, yi = b.y - 1 + o % 3;
-        if (xi < 0 || xi >= N || yi < 0 || yi >= N) continue;
-        const int4* col = a.bins + xi + (long long)yi * N + b.z * NN;
-        const int4 none = make_int4(0, -1, epoch, 0);
-        int4 e = b.z >= 1 && b.z - 1 < N ? col[-NN] : none;
-        int4 e1 = b.z >= 0 && b.z < N ? col[0] : none;
-        int4 e2 = b.z >= -1 && b.z + 1 < N ? col[NN] : none;
+        for (int o = listed.value ? 0 : o0; o < 9; ++o) {
+            const int xi = b.x - 1 + o / 3, yi = b.y - 1 + o % 3;
+            if (xi < 0 || xi >= N || yi < 0 || yi >= N) continue;
+            const int4* col = a.bins + xi + (long long)yi * N + b.z * NN;
+            const int4 none = make_int4(0, -1, epoch, 0);
+            int4 e = b.z >= 1 && b.z - 1 < N ? col[-NN] : none;
+            int4 e1 = b.z >= 0 && b.z < N ? col[0] : none;
+            int4 e2 = b.z >= -1 && b.z + 1 < N ? col[NN] : none;
 #pragma unroll 1
-        for (int z = 0; z < 3; ++z) {
-            const int last = e.z == epoch ? e.y : -1;
+            for (int z = 0; z < 3; ++z) {
+                int last = e.z == epoch ? e.y : -1, j = e.x;
+                if constexpr (!listed.value) {
+                    if (o == o0 && z < z0) last = -1;
+                    if (o == o0 && z == z0 && j < j0) j = j0;
+                }
 #pragma unroll 1
-            for (int j = e.x; j <= last; ++j) {
-                const float4 q = a.cur.posr[j];
-                const uint8_t sj = a.cur.sign[j];
-                const Pair v = pair_of(pr, q);
-                if (v.ss > c.hi || !sj) continue;
-                if (!(v.ss <= c.lo) && pair_dist(v.ss) >= c.t) continue;
-                c = cutoff_bounds(cutoff_of(a, pair_reach(q.w, pr.w)), a.sure);
-                if (v.ss > c.hi) continue;
-                list[cnt][threadIdx.x] = j;
-                if (++cnt == kForceList) work_off();
+                for (; j <= last; ++j) {
+                    const float4 q = a.cur.posr[j];
+                    const uint8_t sj = a.cur.sign[j];
+                    const Pair v = pair_of(pr, q);
+                    if (v.ss > c.hi || !sj) continue;
+                    if (!(v.ss <= c.lo) && pair_dist(v.ss) >= c.t) continue;
+                    const float R = pair_reach(q.w, pr.w);
+                    c = cutoff_bounds(cutoff_of(a, R), a.sure);
+                    if (v.ss > c.hi) continue;
+                    if constexpr (listed.value) {
+                        list[cnt][threadIdx.x] = j;
+                        if (++cnt == kForceList) {
+                            o0 = o;
+                            z0 = z;
+                            j0 = j + 1;
+                            return;
+                        }
+                    } else {
+                        const float d = pair_dist(v.ss);
+                        if (!(d >= c.t)) add(v, d, R, c.t);
+                    }
+                }
+                e = e1;
+                e1 = e2;
             }
-            e = e1;
-            e1 = e2;
         }
+        o0 = 9;
+    };
+    const float cut = cutoff_of(a, pair_reach(pr.w, pr.w)) / a.g.len;
+    const int xf = b.x > 0 ? b.x - 1 : 0, yf = b.y > 0 ? b.y - 1 : 0;
+    const int4 near = inside(xf, yf, b.z, N) ? a.bins[xf + (long long)yf * N + b.z * NN] : make_int4(0, -1, epoch, 0);
+    // (4.19: 4 pi / 3; the count is that of the bins the walk begins with)
+    const bool crowded = near.z == epoch && 4.19f * cut * cut * cut * (float)(near.y - near.x + 1) > (float)kForceCrowd;
+    if (2 * __popc(__ballot_sync(live, crowded)) <= __popc(live)) walk(std::true_type());
+    __syncwarp(live);
+#pragma unroll 1
+    for (int k = 0; k < cnt; ++k) {
+        const float4 q = a.cur.posr[list[k][threadIdx.x]];
+        const Pair v = pair_of(pr, q);
+        const float d = pair_dist(v.ss);
+        const float R = pair_reach(q.w, pr.w);
+        const float own = cutoff_of(a, R);
+        if (!(d >= own)) add(v, d, R, own);
     }
-    work_off();
+    if (o0 < 9) walk(std::false_type());
     live_move(a, i, pr, of, fx, fy, fz);
 }
 
