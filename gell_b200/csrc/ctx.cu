@@ -398,7 +398,7 @@ gell_status gell_create(const gell_params* params, gell_ctx** out) {
     A((void**)&c->bins, (size_t)c->nvox * sizeof(int4));
     A((void**)&c->dev_epoch, sizeof(int));
     A((void**)&c->flags, cap);
-    A((void**)&c->counts, ((cap + 255) / 256) * 4);
+    A((void**)&c->counts, ((cap + 255) / 256 + (cap >> 18) + 1) * 4);
     A((void**)&c->dev_err, 64);
     A((void**)&c->staging, cap * sizeof(gell_cell));
     if (P.rng_mode == GELL_RNG_XORWOW) A((void**)&c->xorwow, cap * sizeof(curandState));
