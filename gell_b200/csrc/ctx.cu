@@ -3,7 +3,6 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 #include <vector>
 #include <cudaTypedefs.h>
 #include <new>
@@ -244,61 +243,25 @@ void gell_substrate_oxygen(gell_substrate* s) {
     s->init = 38.f;
 }
 
-// Pinned words, one per context, into which birth and death write their counts.  A copy to pageable memory
-// costs 12 us a call, and pinning a word of its own 1.7 ms a context: words come from pages of 64 that all
-// contexts share; the first page stays until the process ends, others go when their last word comes back.
-// A page that the runtime no longer knows (the device was reset) is dropped.
-class CountWords {
-public:
-    int* take() {
-        std::lock_guard<std::mutex> lock(m_);
-        for (size_t k = 0; k < pages_.size();) {
-            cudaPointerAttributes at{};
-            if (cudaPointerGetAttributes(&at, pages_[k].base) != cudaSuccess || at.type != cudaMemoryTypeHost) {
-                cudaGetLastError();
-                pages_.erase(pages_.begin() + (long)k);
-                continue;
-            }
-            if (~pages_[k].used) return word(pages_[k]);
-            ++k;
-        }
+struct PinnedPages {
+    static bool known(const int* p) {
+        cudaPointerAttributes at{};
+        const bool ok = cudaPointerGetAttributes(&at, p) == cudaSuccess && at.type == cudaMemoryTypeHost;
+        if (!ok) cudaGetLastError();
+        return ok;
+    }
+    static int* alloc(size_t bytes) {
         void* p = nullptr;
-        if (cudaHostAlloc(&p, 64 * kStride * sizeof(int), cudaHostAllocPortable) != cudaSuccess) return nullptr;
-        pages_.push_back(Page{static_cast<int*>(p), 0});
-        return word(pages_.back());
+        if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return static_cast<int*>(p);
+        cudaGetLastError();
+        return nullptr;
     }
-    void give(int* w) {
-        if (!w) return;
-        std::lock_guard<std::mutex> lock(m_);
-        for (size_t k = 0; k < pages_.size(); ++k) {
-            Page& p = pages_[k];
-            if (w < p.base || w >= p.base + 64 * kStride) continue;
-            p.used &= ~(1ull << ((w - p.base) / kStride));
-            if (!p.used && pages_.size() > 1) {
-                cudaFreeHost(p.base);
-                pages_.erase(pages_.begin() + (long)k);
-            }
-            return;
-        }
+    static void release(int* p) {
+        if (cudaFreeHost(p) != cudaSuccess) cudaGetLastError();
     }
-
-private:
-    static constexpr int kStride = 16;  // 64 bytes a word
-    struct Page {
-        int* base;
-        unsigned long long used;
-    };
-    static int* word(Page& p) {
-        int k = 0;
-        while (p.used >> k & 1) ++k;
-        p.used |= 1ull << k;
-        return p.base + k * kStride;
-    }
-    std::mutex m_;
-    std::vector<Page> pages_;
 };
-static CountWords& count_words() {
-    static CountWords* words = new CountWords;  // never destroyed: contexts may be freed while the process ends
+static CountWords<PinnedPages>& count_words() {
+    static auto* words = new CountWords<PinnedPages>;  // never destroyed: contexts may be freed while the process ends
     return *words;
 }
 
@@ -402,7 +365,7 @@ gell_status gell_create(const gell_params* params, gell_ctx** out) {
     A((void**)&c->dev_err, 64);
     A((void**)&c->staging, cap * sizeof(gell_cell));
     if (P.rng_mode == GELL_RNG_XORWOW) A((void**)&c->xorwow, cap * sizeof(curandState));
-    if (st == GELL_OK && !(c->total = count_words().take())) st = GELL_ERR_CUDA;
+    if (st == GELL_OK && !(c->total = count_words().take()).at) st = GELL_ERR_CUDA;
     if (st != GELL_OK) {
         free_all(c);
         delete c;

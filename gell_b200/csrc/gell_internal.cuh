@@ -23,6 +23,7 @@
 #include <vector>
 
 #include "../../include/gell.h"
+#include "count_words.h"
 
 namespace gell {
 
@@ -148,7 +149,7 @@ struct gell_ctx {
     uint32_t bio_step = 0;
     uint8_t* flags = nullptr;      // cap: cells that divide
     uint32_t* counts = nullptr;    // per 256 or 1,024 cells: how many divide or stay, then sums of 1,024 of those (pd.cu)
-    int* total = nullptr;          // pinned word: their sum, written by the kernel that uses them
+    gell::CountWord total;         // pinned word: their sum, written by the kernel that uses them
     int* dev_err = nullptr;        // device error word (bounded waits)
 
     gell_cell* staging = nullptr;  // cap AoS records

@@ -437,7 +437,7 @@ gell_status birth(gell_ctx* c, int* n_out) {
         a.step = c->bio_step;
         a.flags = c->flags;
         a.counts = c->counts;
-        a.total = c->total;
+        a.total = c->total.at;
         GELL_KERNEL(c, "k_birth_update", launch_dependent(k_birth_update, blocks_for(n, kUpdateCells), kUpdateCells, 0, c->stream, a));
         const bool scanned = blocks_for(n, kUpdateCells) >= kScanFrom;
         if (scanned) {
@@ -447,7 +447,7 @@ gell_status birth(gell_ctx* c, int* n_out) {
             GELL_KERNEL(c, "k_birth_divide", launch_dependent(k_birth_divide<false>, blocks_for(n, kTileCells), kTileCells, 0, c->stream, a));
         }
         GELL_CUDA(c, cudaStreamSynchronize(c->stream));
-        const int total = *c->total;
+        const int total = *c->total.at;
         long long room = (long long)c->cap - 1 - n;
         if (room < 0) room = 0;
         c->n = n + (int)(total < room ? total : room);
@@ -468,9 +468,9 @@ gell_status death(gell_ctx* c, int* n_out) {
         if (scanned)
             if (gell_status st = scan_counts(c, blocks_for(n, kTileCells))) return st;
         GELL_KERNEL(c, "k_compact", launch_dependent((scanned ? k_compact<true> : k_compact<false>), blocks_for(n, kTileCells), kTileCells, 0, c->stream, c->cur(),
-                                                     c->alt(), (const uint32_t*)c->counts, n, c->total));
+                                                     c->alt(), (const uint32_t*)c->counts, n, c->total.at));
         GELL_CUDA(c, cudaStreamSynchronize(c->stream));
-        const int total = *c->total;
+        const int total = *c->total.at;
         c->swap_all();
         c->n = total;
     }
