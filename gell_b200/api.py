@@ -389,7 +389,7 @@ class Simulation:
 
     def set_sweep_warps(self, warps: int) -> None:
         """Line tiles per CTA of the LOD sweeps (0 = as many as fit; the ring sweeps use twice as many
-        warps); results do not change."""
+        warps; the plane sweeps, up to 224^3, have none); results do not change."""
         self._check(self.lib.gell_set_option(self.h, 3, int(warps)), "gell_set_option")
 
     def set_sweep_ring(self, on=True) -> None:
@@ -402,7 +402,8 @@ class Simulation:
         self._check(self.lib.gell_set_option(self.h, 7, int(lag)), "gell_set_option")
 
     def set_lod_streams(self, on: bool = True) -> None:
-        """Each substrate's LOD substeps on a stream of its own (same results)."""
+        """Each substrate's LOD substeps on a stream of its own (the plane sweeps, up to 224^3, take all
+        substrates in one launch; same results)."""
         self._check(self.lib.gell_set_option(self.h, 10, int(bool(on))), "gell_set_option")
 
     def set_sweep_l2hint(self, on: bool = True) -> None:

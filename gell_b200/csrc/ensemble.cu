@@ -6,7 +6,8 @@
 // small kernels of different members run side by side and fill the GPU that any one of them would
 // leave mostly idle.  The graph is replayed for every pair of steps and captured again when a
 // member's cell count, substrates or double-buffer assignment, or the substep count, changed.
-// gell_ensemble_tune times a few branch counts and sweep tile widths and keeps the fastest.
+// gell_ensemble_tune times a few branch counts and, if any member's grid is swept in line tiles, tile
+// widths, and keeps the fastest.
 //
 // Batched (gell_ensemble_set_batched, or chosen by the tuner): each captured step is the FM_update
 // and PreLOD of ALL members as one launch per kernel (gell::mech_batch_step: keys, the sort's
@@ -301,9 +302,12 @@ gell_status gell_ensemble_tune(gell_ensemble* e, int substeps, int* steps_taken,
     int bb = e->branches, bw = e->sweep_warps;
     bool bbat = e->batched;
     gell_status st = GELL_OK;
+    bool line_tiles = false;  // the width is theirs alone
+    for (const gell_ctx* c : e->m) line_tiles = line_tiles || gell::lod_line_tiles(c);
     for (int v = 0; v < 4; ++v) {
         // line-tile widths 0, 2, 1 with per-member sweeps, then the batched sweeps
         const int w = v == 1 ? 2 : (v == 2 ? 1 : 0);
+        if (w != 0 && !line_tiles) continue;
         e->batched = v == 3;
         for (int b = 1; st == GELL_OK; b *= 2) {
             const int br = b < nb ? b : nb;

@@ -293,6 +293,8 @@ inline int blocks_for(long long n, int threads) {
 
 // ------------------------------------------------------------------ entry points between files
 gell_status lod_solver(gell_ctx* c, int sub, int substeps);
+// whether this context's substeps go through line tiles, whose width GELL_OPT_SWEEP_WARPS sets
+bool lod_line_tiles(const gell_ctx* c);
 // LOD substeps of many contexts at once (ensembles): one launch per sweep axis over every member's
 // line tiles.  build allocates the device work list (outside any stream capture); run queues
 // `substeps` substeps of every member on `st`.

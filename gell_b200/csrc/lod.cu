@@ -2035,6 +2035,8 @@ static bool substrate_streams(gell_ctx* c, int s0, int s1) {
     return true;
 }
 
+bool lod_line_tiles(const gell_ctx* c) { return !c->subs.empty() && !planes_by_default(c); }
+
 gell_status lod_solver(gell_ctx* c, int sub, int substeps) {
     if (c->subs.empty() || substeps == 0) return GELL_OK;
     const int s0 = sub < 0 ? 0 : sub, s1 = sub < 0 ? (int)c->subs.size() : sub + 1;

@@ -310,13 +310,14 @@ enum {
  * inputs quantise the change rather than the field.  Weights are trained for one form.
  * GELL_OPT_LOD_STREAMS (0 or 1, default 1): the LOD substeps of each substrate run on a stream of
  * their own (forked from and joined back to the context's stream), so that one substrate's sweep
- * fills the SMs another's leaves idle at its start and end (the plane sweeps take every substrate in
- * one launch instead).  Results are identical. */
+ * fills the SMs another's leaves idle at its start and end (the plane sweeps, N <= 224, take every
+ * substrate in one launch instead).  Results are identical. */
 /* GELL_OPT_CONV_RING: accepted and without effect (the surrogate's convolutions have one form, which
  * passes the input lines through a ring of shared-memory slots). */
 /* GELL_OPT_SWEEP_WARPS (0..4, default 0): line tiles (compute warps) per CTA of the line-tile sweeps;
- * 0 = as many as shared memory holds.  Fewer give more, smaller CTAs, which can fill the GPU
- * better for small grids run side by side (the ensemble tuner tries them).  Results do not change. */
+ * 0 = as many as shared memory holds; without effect on the plane sweeps (N <= 224).  Fewer give
+ * more, smaller CTAs, which can fill the GPU better for grids run side by side (the ensemble tuner
+ * tries them).  Results do not change. */
 gell_status gell_set_option(gell_ctx* ctx, int option, int64_t value);
 
 /*
@@ -362,11 +363,12 @@ gell_status gell_reference_spheroid(const gell_params* p, int n, float cell_radi
  * again when a member's cell count, substrates or buffer assignment, the substep count or the
  * configuration changed.  Each member's own stream is ordered before and after the ensemble's work;
  * biology steps and transfers stay per member (gell_cell_birth / gell_cell_death, ...).
- * gell_ensemble_configure sets the branch count (1..64) and the sweeps' line tiles per CTA
- * (GELL_OPT_SWEEP_WARPS, 0..4) of every member.  gell_ensemble_tune times branch counts 1, 2, 4, ..
- * and tile widths 0, 2, 1, then the batched LOD, with real steps of the members (2 per trial, plus
- * one first step; the total is returned in *steps_taken) and keeps the fastest.  The members must
- * outlive the ensemble and live on the device that is current when it is created.
+ * gell_ensemble_configure sets the branch count (1..64; the batched plane sweeps below take as many
+ * branches as they have groups) and the sweeps' line tiles per CTA (GELL_OPT_SWEEP_WARPS, 0..4) of
+ * every member.  gell_ensemble_tune times branch counts 1, 2, 4, .., for tile widths 0, 2, 1 (only 0
+ * when no member's grid is swept in line tiles) and then for the batched LOD, with real steps of the
+ * members (2 per trial, plus one first step; the total is returned in *steps_taken) and keeps the
+ * fastest.  The members must outlive the ensemble and live on the device that is current when it is created.
  * gell_ensemble_set_batched (0 or 1, default 0): every captured step runs the FM_update and PreLOD
  * of ALL members as one launch per kernel (keys, each radix-sort pass, gather, force and move,
  * uptake map; up to 64 members with up to 4 substrates each, larger ensembles run these on the
