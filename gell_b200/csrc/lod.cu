@@ -338,9 +338,10 @@ __device__ __forceinline__ void forward_uniform(float* slot, int g, int lane, fl
     }
 }
 
-// What bounds it is the chain from one element to the next (one warp per scheduler): two dependent
-// operations since the quotient is taken from a reciprocal in two floats, three before (three sweeps of
-// 400^3 x 2 substrates 0.221 / 0.218 / 0.208 ms before, 0.211 / 0.206 / 0.197 after).
+// The chain from one element to the next is two dependent operations since the quotient is taken from a
+// reciprocal in two floats, three before (three sweeps of 400^3 x 2 substrates 0.221 / 0.218 / 0.208 ms
+// before, 0.211 / 0.206 / 0.197 after).  That gain is the chain's whole share: what bounds the sweep is that a
+// tile stays in shared memory while it is computed, so that few bytes are in flight.
 template <int AXIS>
 __device__ __forceinline__ void backward_uniform(const SubDev& sd, float* slot, int lane, float& x, float o[32],
                                                  int exact) {
@@ -1633,6 +1634,11 @@ gell_status prelod(gell_ctx* c, int sub) {
     return GELL_OK;
 }
 
+static SubDev sub_dev(const Substrate& S, int N) {
+    return SubDev{S.p,         S.rate,  S.line_flag,             S.EF,         S.FRS,    S.s.boundary, S.side, S.uniform_groups,
+                  -S.E[N - 2], -S.side, -(S.side * S.conv_L), -S.F[N - 2], S.conv_R, S.conv_L};
+}
+
 static SrcArgs source_args(const gell_ctx* c, int s0, int s1) {
     SrcArgs sa{};
     for (int s = s0; s < s1; ++s) {
@@ -1761,10 +1767,7 @@ static gell_status lod_solver_range(gell_ctx* c, int s0, int s1, int substeps, c
     int ns = 0;
     for (int s = s0; s < s1; ++s, ++ns) {
         const Substrate& S = c->subs[s];
-        const int N = c->g.N;
-        const SubDev sd{S.p,         S.rate,  S.line_flag,       S.EF,         S.FRS, S.s.boundary,
-                        S.side,      S.uniform_groups,           -S.E[N - 2],  -S.side, -(S.side * S.conv_L), -S.F[N - 2], S.conv_R, S.conv_L};
-        ax.sub[ns] = ay.sub[ns] = az.sub[ns] = axy.sub[ns] = sd;
+        ax.sub[ns] = ay.sub[ns] = az.sub[ns] = axy.sub[ns] = sub_dev(S, c->g.N);
         ax.tm[ns] = S.tmap[0];
         ay.tm[ns] = S.tmap[1];
         az.tm[ns] = S.tmap[2];
@@ -1859,8 +1862,7 @@ gell_status lod_batch_build(const std::vector<gell_ctx*>& ms, LodBatch** out) {
             BatchItem it;
             std::memset(&it, 0, sizeof(it));
             for (int k = 0; k < 3; ++k) it.tm[k] = S.tmap[k];
-                it.sd = SubDev{S.p,    S.rate,           S.line_flag, S.EF,        S.FRS,      S.s.boundary, S.side,
-                           S.uniform_groups, -S.E[N - 2], -S.side, -(S.side * S.conv_L), -S.F[N - 2], S.conv_R, S.conv_L};
+            it.sd = sub_dev(S, N);
             it.g = c->g;
             it.B = B;
             it.exact = c->exact_chain ? 1 : 0;

@@ -84,6 +84,25 @@ static int key_bits(int N) {
     return bits;
 }
 
+static MechArgs mech_args(gell_ctx* c) {
+    MechArgs a;
+    a.cur = c->cur();
+    a.alt = c->alt();
+    a.bins = c->bins;
+    a.epoch = c->dev_epoch;
+    a.n = c->n;
+    a.g = c->g;
+    a.max_dist = c->P.cc_max_dist;
+    a.cccr = c->P.cccr;
+    a.ccca = c->P.ccca;
+    a.ra_ratio = c->P.ra_ratio;
+    a.ra_f = (float)a.ra_ratio;
+    a.ra_exact = (double)a.ra_f == a.ra_ratio;
+    a.sure = a.ra_ratio > 0.0 ? 1.f - 0x1p-18f : -1.f;
+    a.half_dt = c->P.mechanics_dt / 2.f;
+    return a;
+}
+
 static OneJob one_job(gell_ctx* c) {
     return OneJob{c->cur(), c->g, c->sort.keys[0], c->sort.vals[0], c->dev_epoch, c->n, key_bits(c->g.N)};
 }
@@ -105,21 +124,7 @@ gell_status fm_update(gell_ctx* c) {
         GELL_KERNEL(c, "k_gather", launch_dependent(k_gather, blocks_for(n, 256), 256, 0, c->stream, c->cur(), c->alt(), c->sort.keys[w], c->sort.vals[w], n,
                                                               c->bins, c->dev_epoch));
         c->swap_all();
-        MechArgs a;
-        a.cur = c->cur();
-        a.alt = c->alt();
-        a.bins = c->bins;
-        a.epoch = c->dev_epoch;
-        a.n = n;
-        a.g = c->g;
-        a.max_dist = c->P.cc_max_dist;
-        a.cccr = c->P.cccr;
-        a.ccca = c->P.ccca;
-        a.ra_ratio = c->P.ra_ratio;
-        a.ra_f = (float)a.ra_ratio;
-        a.ra_exact = (double)a.ra_f == a.ra_ratio;
-        a.sure = a.ra_ratio > 0.0 ? 1.f - 0x1p-18f : -1.f;
-        a.half_dt = c->P.mechanics_dt / 2.f;
+        const MechArgs a = mech_args(c);
         const int per = force_block(n);
         GELL_KERNEL(c, "k_force_move", launch_dependent((per < kForceThreads ? k_force_warp : k_force_move), blocks_for(n, per), kForceThreads, 0, c->stream, a));
         c->sign.swap();
@@ -418,21 +423,7 @@ gell_status mech_batch_step(const std::vector<gell_ctx*>& ms, cudaStream_t st) {
         const int fblocks = fill_map(fb.map, blocks);
         for (int i = 0; i < nf; ++i) {
             gell_ctx* c = fm[i];
-            MechArgs& a = fb.job[i];
-            a.cur = c->cur();
-            a.alt = c->alt();
-            a.bins = c->bins;
-            a.epoch = c->dev_epoch;
-            a.n = c->n;
-            a.g = c->g;
-            a.max_dist = c->P.cc_max_dist;
-            a.cccr = c->P.cccr;
-            a.ccca = c->P.ccca;
-            a.ra_ratio = c->P.ra_ratio;
-        a.ra_f = (float)a.ra_ratio;
-        a.ra_exact = (double)a.ra_f == a.ra_ratio;
-        a.sure = a.ra_ratio > 0.0 ? 1.f - 0x1p-18f : -1.f;
-            a.half_dt = c->P.mechanics_dt / 2.f;
+            fb.job[i] = mech_args(c);
             c->sign.swap();
             c->mesh.swap();
             c->posr.swap();
