@@ -348,12 +348,6 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv3(const __grid_constant
             nz = w.z1 - w.z0;
         }
         while (ok && u < U) {
-            // a unit of one line leaves its accumulator's hand-over pending, and the next unit's first line
-            // would wait for that accumulator
-            if (m == cacc) {
-                commit();
-                csl = cacc = -1;
-            }
             ok = mbar_wait(&full[sl], gph, a.err, 23);
             if (ok) ok = wait_acc(m, nz);
             if (!ok) break;
@@ -383,6 +377,11 @@ __global__ void __launch_bounds__(kConvThreads, 1) k_conv3(const __grid_constant
             csl = sl;
             cacc = m - 2;
             if (++m == nz + 2) {
+                if (nz == 1) {
+                    // the next unit's first line waits for this very accumulator
+                    commit();
+                    csl = -1;
+                }
                 m = 0;
                 u += gridDim.x;
                 if (u < U) {
