@@ -258,7 +258,9 @@ struct ForceBatch {
     BlockMap map;
     MechArgs job[kBatchMembers];
 };
-__global__ void __launch_bounds__(kForceThreads, 5) k_force_move_batch(const __grid_constant__ ForceBatch b) {
+// (four blocks an SM, 64 registers: with five it spills, since the member's arguments are looked up as well;
+// 24 members of 64^3 to 160^3, two steps 5.168 ms with five, 5.133 with four)
+__global__ void __launch_bounds__(kForceThreads, 4) k_force_move_batch(const __grid_constant__ ForceBatch b) {
     grid_dep_wait();
     grid_dep_launch();
     int local;
