@@ -633,12 +633,36 @@ __device__ __forceinline__ void forward32(const LineCtx& c, int g, int n, float*
     }
 }
 
-// Back substitution of group g from its Y values v: out(k, x) for k = 31 .. 0, as the chain goes.
-// Where any lane's quotient is not the exact one the group is redone on the exact chain and its
-// results are written again.  The factors of a group that is not converged are read four elements
+// Back substitution of the n elements of a group from its Y values w on the exact chain, results to `box`
+// (addressed as elem<ADDR>).  Groups are redone where a line falls through the subnormal numbers (a field that
+// starts at 0 beside a boundary value, with little diffusion), hence 4 elements at a time: by one element a
+// turn cost 140 cycles (10 substeps of 224^3, D = 100 um^2/min from 0: 944 us, 842 so; 131^3, one voxel at 1 in
+// a field of 0, D = 1e4: 528 and 447).  Not inlined: the plane kernel's hot code has to stay in the 32 KB
+// instruction cache, beyond which the issue rate drops by more than half, and inlined it cost 2-4% of a substep.
+template <int ADDR>
+__device__ __noinline__ float redo32(const float4* FR, const float* w, int n, float x, float* box, int lane) {
+#pragma unroll 1
+    for (int q = (n - 1) >> 2; q >= 0; --q) {
+        const float4 y = *reinterpret_cast<const float4*>(w + 4 * q);
+        const float e[4] = {y.x, y.y, y.z, y.w};
+        float4 f[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) f[i] = FR[4 * q + i];
+#pragma unroll
+        for (int i = 3; i >= 0; --i) {
+            x = div_rn(__fmaf_rn(f[i].z, x, e[i]), -f[i].x, f[i].y);
+            *elem<ADDR>(box, 4 * q + i, lane) = x;
+        }
+    }
+    return x;
+}
+
+// Back substitution of group g from its Y values v, results to `box` (addressed as elem<ADDR>) as the
+// chain goes.  Where any lane's quotient is not the exact one the group is redone on the exact chain and
+// its results are written again.  The factors of a group that is not converged are read four elements
 // ahead of their use (a shared load cannot be moved over the results' stores).
-template <class Out>
-__device__ __forceinline__ void backward32(const LineCtx& c, int g, int n, const float* v, float& x, Out out) {
+template <int ADDR>
+__device__ __forceinline__ void backward32(const LineCtx& c, int g, int n, const float* v, float& x, float* box, int lane) {
     const float x_in = x;
     uint32_t bad = 0;
     const bool uni = (c.uni >> g) & 1u;
@@ -647,7 +671,7 @@ __device__ __forceinline__ void backward32(const LineCtx& c, int g, int n, const
         for (int k = 31; k >= 0; --k) {
             const float t = __fmaf_rn(c.nS, x, v[k]);
             x = __fmaf_rn(t, c.R, __fmaf_rn(c.nSL, x, __fmul_rn(v[k], c.L)));
-            out(k, x);
+            *elem<ADDR>(box, k, lane) = x;
             bad |= __float_as_uint(x) ^ __float_as_uint(__fmaf_rn(__fmaf_rn(x, c.nF, t), c.R, x));
         }
     } else {
@@ -666,7 +690,7 @@ __device__ __forceinline__ void backward32(const LineCtx& c, int g, int n, const
                 const int k = 4 * q + i;
                 const float t = __fmaf_rn(f[i].z, x, v[k]);
                 x = __fmaf_rn(t, f[i].y, __fmaf_rn(__fmul_rn(f[i].z, f[i].w), x, __fmul_rn(v[k], f[i].w)));
-                out(k, x);
+                *elem<ADDR>(box, k, lane) = x;
                 bad |= __float_as_uint(x) ^ __float_as_uint(__fmaf_rn(__fmaf_rn(x, f[i].x, t), f[i].y, x));
             }
 #pragma unroll
@@ -674,17 +698,20 @@ __device__ __forceinline__ void backward32(const LineCtx& c, int g, int n, const
         }
     }
     if (__any_sync(FULL, bad != 0) || c.exact) {
-        // rare: a rolled loop over a copy in local memory keeps the kernel small (its hot code has to
-        // stay in the 32 KB instruction cache: beyond it the issue rate drops by more than half)
-        float w[32];
+        alignas(16) float w[32];
 #pragma unroll
         for (int k = 0; k < 32; ++k) w[k] = v[k];
-        x = x_in;
+        if constexpr (ADDR == kSwzCol) {
+            x = redo32<ADDR>(c.FR + 32 * g, w, n < 32 ? n : 32, x_in, box, lane);
+        } else {
+            // (the z tile's kernel has the room for a rolled loop, and was 1% slower at 200^3 with the call)
+            x = x_in;
 #pragma unroll 1
-        for (int k = (n < 32 ? n : 32) - 1; k >= 0; --k) {
-            const float4 f = c.FR[32 * g + k];
-            x = div_rn(__fmaf_rn(f.z, x, w[k]), -f.x, f.y);
-            out(k, x);
+            for (int k = (n < 32 ? n : 32) - 1; k >= 0; --k) {
+                const float4 f = c.FR[32 * g + k];
+                x = div_rn(__fmaf_rn(f.z, x, w[k]), -f.x, f.y);
+                *elem<ADDR>(box, k, lane) = x;
+            }
         }
     }
 }
@@ -757,7 +784,7 @@ __device__ __forceinline__ void plane_body(const CUtensorMap* tm, const SubDev& 
             float* box = rows + (size_t)g * kSlotFloats;
             row_load(box, lane, v);
             __syncwarp();  // every lane has its row: the box takes the results transposed
-            backward32(c, g, N - 32 * g, v, x, [&](int k, float r) { *elem<kSwzCol>(box, k, lane) = r; });
+            backward32<kSwzCol>(c, g, N - 32 * g, v, x, box, lane);
         }
     }
     __syncthreads();
@@ -782,7 +809,7 @@ __device__ __forceinline__ void plane_body(const CUtensorMap* tm, const SubDev& 
             float* box = const_cast<float*>(cols) + (size_t)g * B * kSlotFloats;
             row_load(box, lane, v);
             __syncwarp();  // every lane has its column: the box takes the results as rows again
-            backward32(c, g, N - 32 * g, v, x, [&](int k, float r) { *elem<kSwzCol>(box, k, lane) = r; });
+            backward32<kSwzCol>(c, g, N - 32 * g, v, x, box, lane);
             fence_proxy_async();
             __syncwarp();
             if (lane == 0) {
@@ -856,7 +883,7 @@ __device__ __forceinline__ void ztile_body(const CUtensorMap* tm, const SubDev& 
         float* box = buf + (size_t)g * kSlotFloats;
         row_load(box, lane, v);
         __syncwarp();  // every lane has its Y values: the box takes the results as columns again
-        backward32(c, g, N - 32 * g, v, x, [&](int k, float q) { box[k * 32 + lane] = q; });
+        backward32<2>(c, g, N - 32 * g, v, x, box, lane);
         fence_proxy_async();
         __syncwarp();
         if (lane == 0) {
